@@ -911,9 +911,9 @@ int run_fp32(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b
     p.bias = d->bias; p.bias_is_bf16 = d->bias_dtype == LLMT_B200_BF16;
     p.epi_flags = d->epilogue;
     if (d->batch > 65535) return fail(LLMT_B200_ERR_UNSUPPORTED, "matmul: fp32 path supports batch <= 65535");
-    cudaError_t e = launch_fp32_gemm(p, stream);
-    // The strict-fp32 path has nothing to fuse the bias gradient into: a second small kernel.
-    if (e == cudaSuccess && d->dbias != nullptr) e = launch_fp32_rowsum(p, d->dbias, d->dbias_beta, stream);
+    p.dbias = d->dbias;
+    p.dbias_beta = d->dbias_beta;
+    const cudaError_t e = launch_fp32_gemm(p, stream);
     if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     return LLMT_B200_OK;
 }

@@ -193,6 +193,12 @@ struct Fp32GemmParams {
     const void* bias;
     int32_t bias_is_bf16;
     int32_t epi_flags;
+    float* dbias;               // fp32 [m] or null: dbias[i] = dbias_beta * dbias[i] + sum_k op(A)[i, k]
+    float dbias_beta;
+    // Filled in by launch_fp32_gemm: the launch's tiling and which operands allow 16-byte accesses.
+    int32_t tiles_m, tiles_n, splits;
+    int64_t k_per_split;
+    int32_t vec_a, vec_b, vec_c;
 };
 
 // tanh-GELU in fp32, the expression of llmt's gelu kernel (src/kernels/gelu.cu:23-26).
@@ -271,7 +277,6 @@ int tc_pair_stages(void);
 int tc_dbias_rows_per_cta(void);
 int tc_dbias_finish_per_cta(void);
 cudaError_t launch_fp32_gemm(const Fp32GemmParams& p, cudaStream_t stream);
-cudaError_t launch_fp32_rowsum(const Fp32GemmParams& p, float* dbias, float dbias_beta, cudaStream_t stream);
 cudaError_t launch_zero_f32(float* dst, int64_t n, cudaStream_t stream);
 cudaError_t launch_repack_bf16(void* dst, const void* src, int64_t rows, int64_t cols, int64_t ld_src,
                                int64_t ld_dst, int64_t batch, int64_t stride_src, int64_t stride_dst,
