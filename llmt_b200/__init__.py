@@ -180,9 +180,12 @@ def _check(status: int) -> None:
 
 
 def _stream(stream):
+    """The stream's handle; the current stream of the current device for None (asked of torch without building the
+    Stream object that torch.cuda.current_stream() returns: 3 us)."""
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _dtype_code(t) -> int:
@@ -282,10 +285,8 @@ def plan(desc: GemmDesc) -> str:
 
 def gemm_desc(desc: GemmDesc, c, a, b, stream=None) -> None:
     """Enqueues one llmt_b200_gemm call; `stream` is a torch.cuda.Stream (default: current)."""
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
     _check(lib().llmt_b200_gemm(ctypes.byref(desc), c.data_ptr(), a.data_ptr(), b.data_ptr(),
-                                ctypes.c_void_p(s.cuda_stream)))
+                                _stream(stream)))
 
 
 class Group:
@@ -300,6 +301,7 @@ class Group:
         self.c = (ctypes.c_void_p * n)(*[p[1].data_ptr() for p in problems])
         self.a = (ctypes.c_void_p * n)(*[p[2].data_ptr() for p in problems])
         self.b = (ctypes.c_void_p * n)(*[p[3].data_ptr() for p in problems])
+        self._at = tuple(ctypes.addressof(x) for x in (self.descs, self.c, self.a, self.b))
 
     def workspace_bytes(self):
         out = (ctypes.c_uint64 * self.n)()
@@ -314,20 +316,22 @@ class Group:
                 d.workspace, d.workspace_bytes = buf.data_ptr(), buf.numel()
 
     def run(self, stream=None):
-        import torch
-        s = stream if stream is not None else torch.cuda.current_stream()
-        _check(lib().llmt_b200_gemm_grouped(self.descs, self.c, self.a, self.b, self.n,
-                                            ctypes.c_void_p(s.cuda_stream)))
+        _group_run(*self._at, self.n, stream)
 
     def run_with_exchange(self, comm: "CommDesc", offset: int, count: int, index: int, stream=None):
         """llmt_b200_gemm_grouped_exchange: the same launch, whose epilogue warps also sum floats
         [offset, offset + count) of the gradient span over the ranks through the NVSwitch
         multicast mapping.  The range must be complete before the launch starts."""
-        import torch
-        s = stream if stream is not None else torch.cuda.current_stream()
         _check(lib().llmt_b200_gemm_grouped_exchange(self.descs, self.c, self.a, self.b, self.n, ctypes.byref(comm),
                                                      ctypes.c_int64(int(offset)), ctypes.c_int64(int(count)),
-                                                     ctypes.c_int32(int(index)), ctypes.c_void_p(s.cuda_stream)))
+                                                     ctypes.c_int32(int(index)), _stream(stream)))
+
+
+def _group_run(descs: int, c: int, a: int, b: int, count: int, stream=None) -> None:
+    """llmt_b200_gemm_grouped on arrays given by their addresses."""
+    ptr = ctypes.POINTER(ctypes.c_void_p)
+    _check(lib().llmt_b200_gemm_grouped(ctypes.cast(descs, ctypes.POINTER(GemmDesc)), ctypes.cast(c, ptr),
+                                        ctypes.cast(a, ptr), ctypes.cast(b, ptr), count, _stream(stream)))
 
 
 STATIC_SCRATCH_BYTES = 32 << 20
@@ -338,10 +342,8 @@ def gemm_static_scratch(desc: GemmDesc, c, a, b, stream=None) -> None:
     the fixed array built into the library, so the call allocates nothing and needs no
     workspace from the caller. Problems needing more than STATIC_SCRATCH_BYTES are refused.
     Calls that may overlap on the GPU share (and race on) that one array."""
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
     _check(lib().llmt_b200_gemm_static_scratch(ctypes.byref(desc), c.data_ptr(), a.data_ptr(),
-                                               b.data_ptr(), ctypes.c_void_p(s.cuda_stream)))
+                                               b.data_ptr(), _stream(stream)))
 
 
 def gemm(c, a, b, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, bias=None, gelu=False,
@@ -366,19 +368,15 @@ def gemm(c, a, b, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, bias=None, 
 
 def softmax_fwd(y, x, causal: bool, stream=None) -> None:
     """Row softmax of [batch, Tq, Tk] with llmt's causal rule; y may be x."""
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
     tq, tk = x.shape[-2], x.shape[-1]
     _check(lib().llmt_b200_softmax_fwd(y.data_ptr(), x.data_ptr(), x.numel() // tk, tq, tk,
-                                       _dtype_code(x), int(causal), ctypes.c_void_p(s.cuda_stream)))
+                                       _dtype_code(x), int(causal), _stream(stream)))
 
 
 def softmax_bwd(ds, p, dp, stream=None) -> None:
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
     tk = p.shape[-1]
     _check(lib().llmt_b200_softmax_bwd(ds.data_ptr(), p.data_ptr(), dp.data_ptr(), p.numel() // tk, tk,
-                                       _dtype_code(p), ctypes.c_void_p(s.cuda_stream)))
+                                       _dtype_code(p), _stream(stream)))
 
 
 def head_merge(y, x, stream=None) -> None:
@@ -511,3 +509,28 @@ def set_sm_budget(sms: int) -> int:
 
 def launch_count() -> int:
     return int(lib().llmt_b200_launch_count())
+
+
+# ---- native call path (csrc/pybind.c): the functions above that a program calls many times per step, by their own
+# names; the Python versions stay behind them for whatever they do not recognise.
+
+def _bind_native() -> None:
+    """Gives the native functions the loaded library's entry points (called by the first of them that runs)."""
+    import torch
+    entries = lib()
+    _native.bind(tuple(ctypes.cast(getattr(entries, "llmt_b200_" + n), ctypes.c_void_p).value for n in _native.NAMES),
+                 torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.float32, torch.bfloat16, torch.int32)
+
+
+def _scratch(nbytes: int, like):
+    import torch
+    return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
+
+
+if os.path.exists(os.path.join(_HERE, "_native.so")):
+    from . import _native
+    _native.setup(_bind_native, _check, _scratch)
+    for _f in (_group_run, gemm, gemm_desc, zero_grads, softmax_fwd, softmax_bwd, gemm_softmax_fwd, gemm_softmax_bwd, rowdot,
+               head_split, head_merge, cross_entropy_fwd, cross_entropy_bwd, lm_head_ce_fwd, lm_head_ce_bwd):
+        globals()[_f.__name__] = _native.fast(_f)
+    del _f

@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -78,7 +79,27 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_native(force)
     return LIB_PATH
+
+
+NATIVE_SRC = os.path.join(CSRC, "pybind.c")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
+
+
+def build_native(force: bool = False) -> str:
+    """Builds the CPython extension through which the Python binding makes its frequent calls."""
+    header = os.path.normpath(os.path.join(CSRC, HEADERS[-1]))
+    if force or _stale(NATIVE_PATH, [NATIVE_SRC, header, os.path.abspath(__file__)]):
+        cc = shutil.which("cc") or shutil.which("gcc")
+        if cc is None:
+            raise RuntimeError("a C compiler is required to build llmt_b200/_native.so")
+        cmd = [cc, "-std=c11", "-O2", "-Wall", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], NATIVE_SRC, "-o", NATIVE_PATH]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("the Python extension failed to build")
+    return NATIVE_PATH
 
 
 CPP_DIR = os.path.join(HERE, "cpp")

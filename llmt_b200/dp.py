@@ -17,6 +17,8 @@ from __future__ import annotations
 
 from typing import Dict, Sequence, Tuple
 
+from . import zero_grads
+
 
 def shard_rows(m: int, rank: int, world: int) -> Tuple[int, int]:
     """Contiguous row range [start, stop) of an [m, .] tensor owned by `rank`.
@@ -74,7 +76,6 @@ class GradBucket:
 
     def zero_(self):
         if self.flat.is_cuda:
-            from . import zero_grads
             zero_grads(self.flat)
         else:
             self.flat.zero_()
