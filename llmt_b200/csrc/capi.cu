@@ -637,60 +637,63 @@ Repack repack_plan(const llmt_b200_gemm_desc* d, const Checked& ck, const void* 
     return r;
 }
 
-// Copies the operands that need it behind the split-K region of the workspace and rewrites
-// the (local) descriptor and pointers to use the copies.
-// Copies made for earlier problems of the same grouped launch: an operand that several problems
-// share (dy is the A operand of a layer's dX and of its dW) is copied once.
-struct RepackDone {
-    const void* src;
-    int64_t rows, cols, ld, nb, stride;
-    const void* dst;
-};
-struct RepackCache {
-    RepackDone done[2 * kMaxGroupProblems];
-    int n = 0;
+// The copies a call needs, collected problem by problem and made by one launch before the GEMM's.  An operand that
+// several problems of a grouped launch share (dy is the A operand of a layer's dX and of its dW) is copied once.
+struct RepackList {
+    RepackJobs jobs{};
     const void* find(const void* src, int64_t rows, int64_t cols, int64_t ld, int64_t nb, int64_t stride) const {
-        for (int i = 0; i < n; ++i) {
-            const RepackDone& r = done[i];
-            if (r.src == src && r.rows == rows && r.cols == cols && r.ld == ld && r.nb == nb && r.stride == stride) return r.dst;
+        for (int i = 0; i < jobs.count; ++i) {
+            const RepackJob& r = jobs.job[i];
+            if (r.src == src && r.rows == rows && r.cols == cols && r.ld_src == ld && r.batch == nb && r.stride_src == stride) return r.dst;
         }
         return nullptr;
     }
-    void add(const void* src, int64_t rows, int64_t cols, int64_t ld, int64_t nb, int64_t stride, const void* dst) {
-        if (n < 2 * kMaxGroupProblems) done[n++] = RepackDone{src, rows, cols, ld, nb, stride, dst};
+    int launch(cudaStream_t stream) const {
+        if (jobs.count == 0) return LLMT_B200_OK;
+        const cudaError_t e = launch_repack_bf16(jobs, stream);
+        if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
+        return LLMT_B200_OK;
     }
 };
 
-int apply_repack(llmt_b200_gemm_desc* d, const Checked& ck, const Repack& rp, size_t ws_offset,
-                 const void** a, const void** b, cudaStream_t stream, RepackCache* cache = nullptr) {
+// Adds the copies of the operands that need one to `list` (they go behind the split-K region of the workspace) and
+// rewrites the (local) descriptor and pointers to use the copies.
+void plan_repack(llmt_b200_gemm_desc* d, const Checked& ck, const Repack& rp, size_t ws_offset, const void** a, const void** b,
+                 RepackList* list) {
     char* base = static_cast<char*>(d->workspace) + ws_offset;
     const int64_t nb = d->batch > 1 ? d->batch : 1;
     auto one = [&](const void** src, int64_t rows, int64_t cols, int64_t ld, int64_t stride, int64_t new_ld,
-                   int64_t new_stride, char* dst) -> int {
-        const void* have = cache != nullptr ? cache->find(*src, rows, cols, ld, nb, stride) : nullptr;
+                   int64_t new_stride, char* dst) {
+        const void* have = list->find(*src, rows, cols, ld, nb, stride);
         if (have == nullptr) {
-            cudaError_t e = launch_repack_bf16(dst, *src, rows, cols, ld, new_ld, nb, stride, new_stride, stream);
-            if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
-            if (cache != nullptr) cache->add(*src, rows, cols, ld, nb, stride, dst);
+            RepackJob& r = list->jobs.job[list->jobs.count++];
+            r.dst = reinterpret_cast<uint16_t*>(dst);
+            r.src = static_cast<const uint16_t*>(*src);
+            r.rows = rows; r.cols = cols; r.ld_src = ld; r.ld_dst = new_ld; r.batch = nb; r.stride_src = stride; r.stride_dst = new_stride;
             have = dst;
         }
         *src = have;
-        return LLMT_B200_OK;
     };
     if (rp.a) {
-        const int st = one(a, ck.a_rows, ck.a_cols, d->lda, d->batch > 1 ? d->stride_a : 0, rp.lda, rp.stride_a, base);
-        if (st != LLMT_B200_OK) return st;
+        one(a, ck.a_rows, ck.a_cols, d->lda, d->batch > 1 ? d->stride_a : 0, rp.lda, rp.stride_a, base);
         d->lda = rp.lda;
         d->stride_a = rp.stride_a;
         base += rp.bytes_a;
     }
     if (rp.b) {
-        const int st = one(b, ck.b_rows, ck.b_cols, d->ldb, d->batch > 1 ? d->stride_b : 0, rp.ldb, rp.stride_b, base);
-        if (st != LLMT_B200_OK) return st;
+        one(b, ck.b_rows, ck.b_cols, d->ldb, d->batch > 1 ? d->stride_b : 0, rp.ldb, rp.stride_b, base);
         d->ldb = rp.ldb;
         d->stride_b = rp.stride_b;
     }
-    return LLMT_B200_OK;
+}
+
+// The same for a call of one problem, launched.
+int apply_repack(llmt_b200_gemm_desc* d, const Checked& ck, const Repack& rp, size_t ws_offset,
+                 const void** a, const void** b, cudaStream_t stream) {
+    if (rp.total() == 0) return LLMT_B200_OK;
+    RepackList list;
+    plan_repack(d, ck, rp, ws_offset, a, b, &list);
+    return list.launch(stream);
 }
 
 int check_workspace(const llmt_b200_gemm_desc* d, const TcPlan& pl, size_t repack_bytes = 0) {
@@ -832,6 +835,11 @@ int launch_group(GroupProblem* probs, int count, bool pairs, cudaStream_t stream
         else gp.ride.tiles = 0;
         gp.ride_counter = g->ride_counters + slot;
         gp.total_tiles = static_cast<int32_t>(total);
+        int widest = 0;
+        for (int i = 0; i < n; ++i) widest = gp.prob[i].bn > widest ? gp.prob[i].bn : widest;
+        gp.stages = tc_stages(pairs, widest);
+        gp.stage_bytes = tc_stage_bytes(pairs, widest);
+        gp.inv_stages = 1.0f / static_cast<float>(gp.stages);
         gp.sched_counter = g->counters + slot;
         gp.dbias_sync = g->dbias_sync + 2 * slot;
         gp.static_schedule = static_schedule_forced() ? 1 : 0;
@@ -1056,7 +1064,7 @@ int gemm_grouped_impl(const llmt_b200_gemm_desc* descs, void* const* c, const vo
                         "gemm_grouped: problem %d asks for CTA pairs, but another problem of the launch cannot run "
                         "on pairs (a launch is all pairs or all single CTAs)", i);
     GroupProblem probs[kMaxGroupProblems];
-    RepackCache repacked;
+    RepackList repacked;
     int n = 0;
     for (int i = 0; i < count; ++i) {
         if (descs[i].m == 0 || descs[i].n == 0 || descs[i].batch == 0) continue;
@@ -1069,15 +1077,13 @@ int gemm_grouped_impl(const llmt_b200_gemm_desc* descs, void* const* c, const vo
         llmt_b200_gemm_desc local = descs[i];
         const void* ai = a[i];
         const void* bi = b[i];
-        if (rp.total() > 0) {
-            st = apply_repack(&local, ck[i], rp, plans[i].workspace_bytes, &ai, &bi,
-                              static_cast<cudaStream_t>(stream), &repacked);
-            if (st != LLMT_B200_OK) return st;
-        }
+        if (rp.total() > 0) plan_repack(&local, ck[i], rp, plans[i].workspace_bytes, &ai, &bi, &repacked);
         st = fill_problem(&probs[n], &local, ck[i], plans[i], c[i], ai, bi);
         if (st != LLMT_B200_OK) return st;
         ++n;
     }
+    const int rst = repacked.launch(static_cast<cudaStream_t>(stream));
+    if (rst != LLMT_B200_OK) return rst;
     if (comm == nullptr) {
         if (n == 0) return LLMT_B200_OK;
         return launch_group(probs, n, pairs, static_cast<cudaStream_t>(stream));
@@ -1125,10 +1131,11 @@ bool is_tc_problem(const llmt_b200_gemm_desc& d) {
 
 namespace {
 // Layout of the workspace of llmt_b200_lm_head_ce_fwd: the GEMM's own scratch (repacked operands),
-// then the per-part (maximum, sum of exponentials) pairs, then the target logits.
+// then the per-part (maximum, sum of exponentials) pairs, the target logits, the backward epilogue's row
+// values and the rows' log-sum-exp.
 struct LmHeadCePlan {
     TcPlan pl;
-    size_t gemm_bytes, stats_off, tgt_off, grad_off, sum_off, total;
+    size_t gemm_bytes, stats_off, tgt_off, grad_off, lse_off, total;
     int parts;
 };
 // One plan for the forward and the backward call on the same product, whatever type each of them
@@ -1144,8 +1151,8 @@ LmHeadCePlan lm_head_ce_plan(const llmt_b200_gemm_desc* d, const Checked& ck, co
     r.stats_off = (r.gemm_bytes + 255) / 256 * 256;
     r.tgt_off = r.stats_off + (static_cast<size_t>(r.parts) * d->m * 8 + 255) / 256 * 256;
     r.grad_off = r.tgt_off + (static_cast<size_t>(d->m) * 4 + 255) / 256 * 256;    // (lse, weight) per row
-    r.sum_off = r.grad_off + (static_cast<size_t>(d->m) * 8 + 255) / 256 * 256;    // the mask's sum
-    r.total = r.sum_off + 256;
+    r.lse_off = r.grad_off + (static_cast<size_t>(d->m) * 8 + 255) / 256 * 256;    // the rows' log-sum-exp, left by the forward call
+    r.total = r.lse_off + (static_cast<size_t>(d->m) * 4 + 255) / 256 * 256;
     return r;
 }
 int lm_head_ce_check(const llmt_b200_gemm_desc* d) {
@@ -1202,7 +1209,9 @@ int llmt_b200_lm_head_ce_fwd(const llmt_b200_gemm_desc* d, void* logits, const v
     p.epi_flags |= kEpiLse;
     st = launch_group(&p, 1, lp.pl.pairs != 0, s, nullptr, /*lse=*/true);
     if (st != LLMT_B200_OK) return st;
-    cudaError_t e = launch_cross_entropy_from_stats(loss, row_nll, p.ext_stats, p.ext_rowvec, mask, d->m, lp.parts, s);
+    cudaError_t e = launch_ce_from_stats(row_nll, reinterpret_cast<float*>(ws + lp.lse_off), p.ext_stats, p.ext_rowvec, mask, d->m,
+                                         lp.parts, s);
+    if (e == cudaSuccess) e = launch_ce_mean(loss, row_nll, mask, d->m, s);
     if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     return LLMT_B200_OK;
 }
@@ -1247,8 +1256,10 @@ int llmt_b200_lm_head_ce_bwd(const llmt_b200_gemm_desc* d, void* dlogits, const 
         if (st != LLMT_B200_OK) return st;
     }
     float2* rows = reinterpret_cast<float2*>(ws + lp.grad_off);
-    cudaError_t e = launch_ce_grad_rows(rows, stats, nullptr, mask, reinterpret_cast<float*>(ws + lp.sum_off), dloss,
-                                        d->m, lp.parts, s);
+    float* lse = reinterpret_cast<float*>(ws + lp.lse_off);
+    cudaError_t e = cudaSuccess;
+    if (!stats_valid) e = launch_ce_from_stats(nullptr, lse, stats, nullptr, nullptr, d->m, lp.parts, s);
+    if (e == cudaSuccess) e = launch_ce_grad_rows(rows, lse, mask, dloss, d->m, s);
     if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     st = fill_problem(&p, &local, ck, lp.pl, dlogits, a, b);
     if (st != LLMT_B200_OK) return st;
@@ -1478,7 +1489,7 @@ int llmt_b200_gemm_plan(const llmt_b200_gemm_desc* d, char* buf, size_t n) {
     const int units = pl.pairs ? pair_units() : sm_count();
     const int64_t tickets = pl.num_tiles + pl.colsum_tiles + pl.fin_tiles;
     snprintf(buf, n, "tcgen05 %s tile=%dx%dx64 stages=%d splits=%d tiles=%dx%d kblocks=%d dbias_tickets=%d grid=%d smem=%zu ws=%zu resident_pairs=%d",
-             pl.pairs ? "cta-pair" : "1-cta", pl.pairs ? 256 : 128, pl.bn, pl.pairs ? tc_pair_stages() : 4, pl.splits, pl.tiles_m,
+             pl.pairs ? "cta-pair" : "1-cta", pl.pairs ? 256 : 128, pl.bn, tc_stages(pl.pairs != 0, pl.bn), pl.splits, pl.tiles_m,
              pl.tiles_n, pl.kblocks_total, pl.colsum_tiles + pl.fin_tiles,
              static_cast<int>(tickets < units ? tickets : units) * (pl.pairs ? 2 : 1),
              tc_grouped_smem_bytes(), pl.workspace_bytes, pl.pairs ? max_resident_pairs() : 0);

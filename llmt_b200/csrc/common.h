@@ -135,6 +135,9 @@ struct GroupParams {
     int32_t fin_begin;          // tickets [fin_begin, total_tiles) finish the two-phase dbias reductions
     int32_t* dbias_sync;        // [2] arrival counters of the two phases; zero between launches
     int32_t static_schedule;    // 1 = ticket i goes to CTA i % grid instead of the dynamic queue
+    int32_t stages;             // operand stages in shared memory, sized for the widest tile of the launch
+    uint32_t stage_bytes;
+    float inv_stages;
     int32_t* sched_counter;     // zero between launches; the kernel re-arms it
     DeviceStatus* status;
     uint64_t wait_limit_ns;     // every wait inside the kernel gives up after this long
@@ -199,6 +202,22 @@ struct Fp32GemmParams {
     int32_t tiles_m, tiles_n, splits;
     int64_t k_per_split;
     int32_t vec_a, vec_b, vec_c;
+};
+
+// Copies of operands that TMA cannot address, one launch for all of a call's (see repack_bf16_kernel).
+struct RepackJob {
+    uint16_t* dst;
+    const uint16_t* src;
+    int64_t rows, cols, ld_src, ld_dst, batch, stride_src, stride_dst;
+    // Filled in by launch_repack_bf16:
+    int64_t total_rows;      // rows * batch
+    uint32_t lanes, strips;  // threads along a row; blocks side by side that cover a long one
+    uint32_t first_block;
+};
+constexpr int kMaxRepacks = 2 * kMaxGroupProblems;
+struct RepackJobs {
+    RepackJob job[kMaxRepacks];
+    int32_t count;
 };
 
 // tanh-GELU in fp32, the expression of llmt's gelu kernel (src/kernels/gelu.cu:23-26).
@@ -268,19 +287,19 @@ __device__ __forceinline__ float dgelu_tanh_precise(float x) {
 cudaError_t launch_tc_grouped(const GroupParams& gp, int grid, bool pairs, cudaStream_t stream, bool lse = false);
 cudaError_t launch_cross_entropy_fwd(float* loss, float* row_nll, const float* logits, const int32_t* targets,
                                      const float* mask, int64_t rows, int64_t v, int64_t ld, cudaStream_t stream);
-cudaError_t launch_cross_entropy_from_stats(float* loss, float* row_nll, const void* stats, const float* tgt,
-                                            const float* mask, int64_t rows, int parts, cudaStream_t stream);
+cudaError_t launch_ce_from_stats(float* row_nll, float* lse, const void* stats, const float* tgt, const float* mask, int64_t rows,
+                                 int parts, cudaStream_t stream);
+cudaError_t launch_ce_mean(float* loss, const float* row_nll, const float* mask, int64_t rows, cudaStream_t stream);
 int max_resident_pairs(void);
 cudaError_t launch_splitk_reduce(const GroupProblem& p, cudaStream_t stream);
 size_t tc_grouped_smem_bytes(void);
-int tc_pair_stages(void);
+uint32_t tc_stage_bytes(bool pairs, int bn);   // one operand stage of a launch whose widest tile is bn
+int tc_stages(bool pairs, int bn);             // and how many of them a CTA has
 int tc_dbias_rows_per_cta(void);
 int tc_dbias_finish_per_cta(void);
 cudaError_t launch_fp32_gemm(const Fp32GemmParams& p, cudaStream_t stream);
 cudaError_t launch_zero_f32(float* dst, int64_t n, cudaStream_t stream);
-cudaError_t launch_repack_bf16(void* dst, const void* src, int64_t rows, int64_t cols, int64_t ld_src,
-                               int64_t ld_dst, int64_t batch, int64_t stride_src, int64_t stride_dst,
-                               cudaStream_t stream);
+cudaError_t launch_repack_bf16(RepackJobs jobs, cudaStream_t stream);
 cudaError_t launch_softmax_fwd(void* y, const void* x, int64_t rows, int64_t tq, int64_t tk,
                                int is_bf16, int causal, cudaStream_t stream);
 cudaError_t launch_softmax_bwd(void* ds, const void* p, const void* dp, int64_t rows, int64_t tk,
@@ -292,13 +311,30 @@ cudaError_t launch_head_split(void* q, void* k, void* v, const void* qkv, int64_
 cudaError_t launch_cross_entropy_bwd(float* dlogits, const float* logits, const int32_t* targets, const float* mask,
                                      float dloss, int64_t rows, int64_t v, int64_t ld_in, int64_t ld_out,
                                      cudaStream_t stream);
-cudaError_t launch_ce_grad_rows(void* out, const void* stats, const float* lse_in, const float* mask, float* mask_sum,
-                                float dloss, int64_t rows, int parts, cudaStream_t stream);
+cudaError_t launch_ce_grad_rows(void* out, const float* lse, const float* mask, float dloss, int64_t rows, cudaStream_t stream);
 cudaError_t launch_lse_from_stats(float* lse, const void* stats, int64_t rows, int parts, cudaStream_t stream);
 cudaError_t launch_rowdot(float* out, const void* x, const void* y, int64_t rows, int64_t cols, int64_t ldx,
                           int64_t ldy, int is_bf16, cudaStream_t stream);
 DeviceStatus* device_status_ptr(void);
 
 void count_launch(int n);
+
+// Launches a kernel as a programmatic dependent of the one before it in the stream: its blocks may start while that one
+// drains, and wait (griddepcontrol.wait, which every kernel launched this way executes first) before they touch memory.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    count_launch(1);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
 
 }  // namespace llmt_b200

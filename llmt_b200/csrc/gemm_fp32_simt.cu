@@ -389,11 +389,87 @@ __device__ __forceinline__ MaxSum merge(MaxSum a, MaxSum b) {
 
 // Row softmax with llmt's masking rule (src/kernels/softmax.cu:33-50: under the causal mask
 // only columns <= r % tq take part; the others are written as exact zeros; y may be x).
-// One warp per row, ONE pass over the scores to find (max, sum) - each lane keeps a running
-// pair that is rescaled whenever its maximum grows, the 32 pairs merge in a butterfly - and
-// one pass to write, instead of llmt's three passes.
+// Bound: HBM, one read and one write of the scores.  One warp per row.  Rows of up to 32 * N values are
+// held in registers (N per lane, 16-byte accesses where VEC says the rows allow them): one read, one
+// exponential per value, one write.  Longer rows take one pass to find (max, sum), each lane keeping
+// a running pair that is rescaled whenever its maximum grows, and one to write.
+template <typename T, int N, bool VEC>
+__global__ void __launch_bounds__(128)
+softmax_rows_kernel(T* y, const T* x, int64_t rows, int64_t tq, int64_t tk, int causal) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (r >= rows) return;
+    const int live = static_cast<int>(causal ? (r % tq) + 1 : tk);  // columns that take part
+    const T* in = x + r * tk;
+    T* out = y + r * tk;
+    constexpr int kPer = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;   // consecutive values per access
+    float v[N];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < N / kPer; ++i) {
+        const int c = (i * 32 + lane) * kPer;
+        float* to = v + i * kPer;
+        if (VEC) {
+            uint4 w = make_uint4(0, 0, 0, 0);
+            if (c < live) w = *reinterpret_cast<const uint4*>(in + c);
+            const uint32_t q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (sizeof(T) == 4) {
+                    to[j] = __uint_as_float(q[j]);
+                } else {
+                    to[(2 * j) % kPer] = __uint_as_float(q[j] << 16);
+                    to[(2 * j + 1) % kPer] = __uint_as_float(q[j] & 0xFFFF0000u);
+                }
+            }
+        } else if (c < live) {
+            to[0] = Elem<T>::get(in, c);
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (c + j >= live) to[j] = -INFINITY;
+            mx = fmaxf(mx, to[j]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        v[i] = expf(v[i] - mx);   // exp(-inf) = 0: absent columns
+        sum += v[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float scale = 1.0f / sum;
+#pragma unroll
+    for (int i = 0; i < N / kPer; ++i) {
+        const int c = (i * 32 + lane) * kPer;
+        if (c >= tk) break;
+        const float* from = v + i * kPer;
+        if (VEC) {
+            uint32_t q[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (sizeof(T) == 4) {
+                    q[j] = __float_as_uint(from[j] * scale);
+                } else {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(from[(2 * j) % kPer] * scale, from[(2 * j + 1) % kPer] * scale);
+                    q[j] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+            }
+            *reinterpret_cast<uint4*>(out + c) = make_uint4(q[0], q[1], q[2], q[3]);
+        } else {
+            Elem<T>::put(out, c, from[0] * scale);
+        }
+    }
+}
+
 template <typename T>
-__global__ void softmax_rows_kernel(T* y, const T* x, int64_t rows, int64_t tq, int64_t tk, int causal) {
+__global__ void __launch_bounds__(128)
+softmax_long_rows_kernel(T* y, const T* x, int64_t rows, int64_t tq, int64_t tk, int causal) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (r >= rows) return;
@@ -424,7 +500,10 @@ __global__ void softmax_rows_kernel(T* y, const T* x, int64_t rows, int64_t tq, 
 
 // dS = P * (dP - sum_c dP[c] P[c]) per row (llmt docs/TODO.md:227).  ds may be dp.
 template <typename T>
-__global__ void softmax_rows_bwd_kernel(T* ds, const T* p, const T* dp, int64_t rows, int64_t tk) {
+__global__ void __launch_bounds__(128)
+softmax_rows_bwd_kernel(T* ds, const T* p, const T* dp, int64_t rows, int64_t tk) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (r >= rows) return;
@@ -439,79 +518,130 @@ __global__ void softmax_rows_bwd_kernel(T* ds, const T* p, const T* dp, int64_t 
         Elem<T>::put(out, c, Elem<T>::get(pr, c) * (Elem<T>::get(gr, c) - dot));
 }
 
-// Copies a row-major bf16 matrix (any pitch, any 2-byte alignment) into a buffer whose base is
-// 16-byte aligned and whose pitch is a multiple of 8 elements, so that TMA can address it.
-// One thread per 8 output elements (one 16-byte store): the source elements come from the
-// five aligned 32-bit words that cover them, shifted by 16 bits when the source row starts on
-// an odd element.  Columns beyond `cols` are written as zeros.
-__global__ void repack_bf16_kernel(uint16_t* __restrict__ dst, const uint16_t* __restrict__ src, int64_t rows,
-                                   int64_t cols, int64_t ld_src, int64_t ld_dst, int64_t batch,
-                                   int64_t stride_src, int64_t stride_dst) {
-    const int64_t groups_per_row = ld_dst / 8;
-    const int64_t total = batch * rows * groups_per_row;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t g = i % groups_per_row;
-        const int64_t r = (i / groups_per_row) % rows;
-        const int64_t b = i / (groups_per_row * rows);
-        const int64_t c0 = g * 8;
-        const uint16_t* s = src + b * stride_src + r * ld_src + c0;
-        uint32_t out[4];
-        if (c0 + 8 <= cols) {
-            const uintptr_t addr = reinterpret_cast<uintptr_t>(s);
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(addr & ~static_cast<uintptr_t>(3));
-            if ((addr & 2u) == 0u) {
+// Copies row-major bf16 matrices (any pitch, any 2-byte alignment) into buffers whose base is
+// 16-byte aligned and whose pitch is a multiple of 8 elements, so that TMA can address them: up to
+// kMaxRepacks of them in one launch (the operands of a grouped GEMM call).  Columns beyond `cols` are
+// written as zeros.  Bound: HBM (8192 x 50257: 823 MB in, 823 MB out), which leaves a warp about 80
+// instructions per 16-byte group: with a division and a row's address per group the copy took 430 us, so a
+// thread's groups (kRepackUnits, all in flight) lie at fixed distances from one address.  The source's
+// bytes come from the one or two aligned 16-byte words that cover them, shifted by the row's offset; the
+// second word is the next lane's first and comes from it.
+constexpr int kRepackUnits = 4;
+
+__device__ __forceinline__ uint4 repack_shift(const uint4& lo, const uint4& hi, uint32_t off) {
+    uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    if (off & 8u) { w[0] = w[2]; w[1] = w[3]; w[2] = w[4]; w[3] = w[5]; w[4] = w[6]; w[5] = w[7]; }
+    if (off & 4u) { w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = w[4]; w[4] = w[5]; }
+    if (off & 2u) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) out[j] = w[j];
-            } else {
-                uint32_t v[5];
+        for (int j = 0; j < 4; ++j) w[j] = __funnelshift_r(w[j], w[j + 1], 16);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// The last group of a row: `left` (< 8) values, then zeros.
+__device__ __forceinline__ uint4 repack_tail(const uint16_t* s, int left) {
+    uint32_t q[4];
 #pragma unroll
-                for (int j = 0; j < 5; ++j) v[j] = w[j];   // the first and last halves belong to neighbours
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t x = 2 * j < left ? s[2 * j] : 0u, y = 2 * j + 1 < left ? s[2 * j + 1] : 0u;
+        q[j] = x | (y << 16);
+    }
+    return make_uint4(q[0], q[1], q[2], q[3]);
+}
+
+__global__ void __launch_bounds__(256)
+repack_bf16_kernel(const __grid_constant__ RepackJobs jobs) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int ji = 0;
+    while (ji + 1 < jobs.count && blockIdx.x >= jobs.job[ji + 1].first_block) ++ji;
+    const RepackJob& p = jobs.job[ji];
+    const uint32_t block = blockIdx.x - p.first_block;
+    const uint32_t strip = block % p.strips, chunk = block / p.strips;
+    // A block takes `lanes` threads along a row and 256 / lanes rows at a time.  Long rows (all 256 threads): the units
+    // follow each other along the row, `strips` blocks side by side.  Short rows: the units are consecutive runs of rows.
+    const int shift = __ffs(static_cast<int>(p.lanes)) - 1;
+    const bool along = p.lanes == 256u;
+    const int lane_g = static_cast<int>(threadIdx.x & (p.lanes - 1u));
+    const int64_t row0 = along ? chunk : static_cast<int64_t>(chunk) * ((256u >> shift) * kRepackUnits) + (threadIdx.x >> shift);
+    const int64_t dr = along ? 0 : 256 >> shift;
+    const int64_t c0 = 8 * (static_cast<int64_t>(strip) * (256 * kRepackUnits) + lane_g);
+    const int dc = along ? 8 * 256 : 0;
+    const bool last_lane = (threadIdx.x & 31u) == 31u;
+    uint4 lo[kRepackUnits], hi[kRepackUnits];
+    const uint16_t* src[kRepackUnits];
+    uint16_t* dst[kRepackUnits];
+    int left[kRepackUnits];   // values of the row from the unit on; <= -8: nothing to write
 #pragma unroll
-                for (int j = 0; j < 4; ++j) out[j] = __funnelshift_r(v[j], v[j + 1], 16);
-            }
+    for (int i = 0; i < kRepackUnits; ++i) {
+        if (i == 0 || !along) {
+            const int64_t row = row0 + i * dr;   // over the rows of all batch items
+            const int64_t b = p.batch > 1 ? row / p.rows : 0, r = row - b * p.rows;
+            src[i] = p.src + b * p.stride_src + r * p.ld_src + c0;
+            dst[i] = p.dst + b * p.stride_dst + r * p.ld_dst + c0;
+            left[i] = row < p.total_rows && c0 < p.ld_dst ? static_cast<int>(p.cols - c0) : -8;
         } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t lo = c0 + 2 * j < cols ? s[2 * j] : 0u;
-                const uint32_t hi = c0 + 2 * j + 1 < cols ? s[2 * j + 1] : 0u;
-                out[j] = lo | (hi << 16);
-            }
+            src[i] = src[0] + i * dc;
+            dst[i] = dst[0] + i * dc;
+            left[i] = left[0] - i * dc;
         }
-        *reinterpret_cast<uint4*>(dst + b * stride_dst + r * ld_dst + c0) = make_uint4(out[0], out[1], out[2], out[3]);
+        lo[i] = hi[i] = make_uint4(0, 0, 0, 0);
+        if (left[i] >= 8) {
+            const uintptr_t at = reinterpret_cast<uintptr_t>(src[i]);
+            const uint4* w = reinterpret_cast<const uint4*>(at & ~static_cast<uintptr_t>(15));
+            lo[i] = __ldg(w);
+            if ((at & 15u) != 0 && (last_lane || left[i] < 16)) hi[i] = __ldg(w + 1);
+        } else if (left[i] > 0) {
+            lo[i] = repack_tail(src[i], left[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kRepackUnits; ++i) {
+        const uint4 next = make_uint4(__shfl_down_sync(0xffffffffu, lo[i].x, 1), __shfl_down_sync(0xffffffffu, lo[i].y, 1),
+                                      __shfl_down_sync(0xffffffffu, lo[i].z, 1), __shfl_down_sync(0xffffffffu, lo[i].w, 1));
+        if (left[i] <= -8) continue;
+        const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src[i]) & 15u);
+        uint4 v = lo[i];
+        if (left[i] >= 8 && off != 0) v = repack_shift(lo[i], !last_lane && left[i] >= 16 ? next : hi[i], off);
+        *reinterpret_cast<uint4*>(dst[i]) = v;
     }
 }
 
 // Head split / merge as copies (llmt include/llmt/kernels/permute.h:21-46).  The GEMMs can read
 // and write the per-head layout through strides, so these are only needed where a caller wants
-// the re-shelved tensor itself.  One thread moves `vec` consecutive elements of one head's row
+// the re-shelved tensor itself.  A block takes one token row at a time (no 64-bit division per element: that
+// bound the kernel at 9 us for 9.4 MB), a thread moves `vec` consecutive elements of one head's row
 // (hd is a multiple of vec): 16 bytes when the pointers and hd allow it, else one element.
 //   merge: y[b, t, h*hd + d] = x[b, h, t, d]
 //   split: out[part][b, h, t, d] = qkv[b, t, part*A + h*hd + d],  A = H*hd, part = 0..parts-1
 template <typename V>
-__global__ void head_merge_kernel(V* __restrict__ y, const V* __restrict__ x, int64_t B, int64_t H, int64_t T,
-                                  int64_t hdv) {
-    const int64_t total = B * H * T * hdv;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        // i runs over the OUTPUT [B, T, H, hdv]: consecutive threads write consecutive vectors
-        const int64_t d = i % hdv, h = (i / hdv) % H, t = (i / (hdv * H)) % T, b = i / (hdv * H * T);
-        y[i] = x[((b * H + h) * T + t) * hdv + d];
+__global__ void __launch_bounds__(256)
+head_merge_kernel(V* __restrict__ y, const V* __restrict__ x, int64_t tokens, uint32_t H, int64_t T, uint32_t hdv) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t width = H * hdv;
+    for (int64_t token = blockIdx.x; token < tokens; token += gridDim.x) {
+        const int64_t b = token / T, t = token - b * T;
+        for (uint32_t i = threadIdx.x; i < width; i += 256u) {
+            const uint32_t h = i / hdv, d = i - h * hdv;
+            y[token * width + i] = x[((b * H + h) * T + t) * hdv + d];
+        }
     }
 }
 
 template <typename V>
-__global__ void head_split_kernel(V* __restrict__ q, V* __restrict__ k, V* __restrict__ v, const V* __restrict__ qkv,
-                                  int64_t B, int64_t H, int64_t T, int64_t hdv) {
-    const int64_t per_part = B * T * H * hdv;
-    const int64_t total = 3 * per_part;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        // i runs over the INPUT [B, T, 3, H, hdv]: consecutive threads read consecutive vectors
-        const int64_t d = i % hdv, h = (i / hdv) % H, part = (i / (hdv * H)) % 3, t = (i / (hdv * H * 3)) % T,
-                      b = i / (hdv * H * 3 * T);
-        V* out = part == 0 ? q : part == 1 ? k : v;
-        out[((b * H + h) * T + t) * hdv + d] = qkv[i];
+__global__ void __launch_bounds__(256)
+head_split_kernel(V* __restrict__ q, V* __restrict__ k, V* __restrict__ v, const V* __restrict__ qkv, int64_t tokens, uint32_t H, int64_t T,
+                  uint32_t hdv) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t width = H * hdv;
+    for (int64_t token = blockIdx.x; token < tokens; token += gridDim.x) {
+        const int64_t b = token / T, t = token - b * T;
+        for (uint32_t i = threadIdx.x; i < 3u * width; i += 256u) {
+            const uint32_t head = i / hdv, d = i - head * hdv;   // over the heads of q, k and v
+            const uint32_t part = head / H, h = head - part * H;
+            V* out = part == 0 ? q : part == 1 ? k : v;
+            out[((b * H + h) * T + t) * hdv + d] = qkv[token * (3 * static_cast<int64_t>(width)) + i];
+        }
     }
 }
 
@@ -559,18 +689,22 @@ cudaError_t launch_zero_f32(float* dst, int64_t n, cudaStream_t stream) {
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-cudaError_t launch_repack_bf16(void* dst, const void* src, int64_t rows, int64_t cols, int64_t ld_src,
-                               int64_t ld_dst, int64_t batch, int64_t stride_src, int64_t stride_dst,
-                               cudaStream_t stream) {
-    const int64_t total = batch * rows * (ld_dst / 8);   // ld_dst is a multiple of 8
-    int64_t grid = (total + 255) / 256;
-    if (grid > 148 * 32) grid = 148 * 32;
-    if (grid < 1) grid = 1;
-    repack_bf16_kernel<<<static_cast<unsigned>(grid), 256, 0, stream>>>(
-        static_cast<uint16_t*>(dst), static_cast<const uint16_t*>(src), rows, cols, ld_src, ld_dst, batch,
-        stride_src, stride_dst);
-    count_launch(1);
-    return cudaGetLastError();
+cudaError_t launch_repack_bf16(RepackJobs jobs, cudaStream_t stream) {
+    int64_t blocks = 0;
+    for (int i = 0; i < jobs.count; ++i) {
+        RepackJob& p = jobs.job[i];
+        const int64_t groups = p.ld_dst / 8;   // ld_dst is a multiple of 8
+        uint32_t lanes = 1;                    // threads along a row: a power of two, so that short rows share a block
+        while (lanes < 256 && lanes < groups) lanes *= 2;
+        p.lanes = lanes;
+        p.strips = lanes == 256 ? static_cast<uint32_t>((groups + 256 * kRepackUnits - 1) / (256 * kRepackUnits)) : 1;
+        p.total_rows = p.rows * p.batch;
+        p.first_block = static_cast<uint32_t>(blocks);
+        const int64_t rows_per_block = lanes == 256 ? 1 : static_cast<int64_t>(256 / lanes) * kRepackUnits;
+        blocks += (p.total_rows + rows_per_block - 1) / rows_per_block * p.strips;
+        if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+    }
+    return launch_dependent(repack_bf16_kernel, static_cast<unsigned>(blocks), 256, stream, jobs);
 }
 
 namespace {
@@ -668,84 +802,72 @@ cudaError_t launch_fp32_gemm(const Fp32GemmParams& in, cudaStream_t stream) {
 }
 
 namespace {
-int64_t copy_grid(int64_t total) {
-    int64_t grid = (total + 255) / 256;
-    if (grid > 148 * 16) grid = 148 * 16;
-    return grid < 1 ? 1 : grid;
-}
 bool vec16_ok(std::initializer_list<const void*> ptrs, int64_t hd, int elem_bytes) {
     if ((hd * elem_bytes) % 16 != 0) return false;
     for (const void* p : ptrs)
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;
     return true;
 }
+unsigned token_blocks(int64_t tokens) { return static_cast<unsigned>(tokens < 148 * 64 ? tokens : 148 * 64); }
+
+template <typename V>
+cudaError_t head_merge_as(void* y, const void* x, int64_t B, int64_t H, int64_t T, int64_t hdv, cudaStream_t stream) {
+    return launch_dependent(head_merge_kernel<V>, token_blocks(B * T), 256, stream, static_cast<V*>(y), static_cast<const V*>(x), B * T,
+                            static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv));
+}
+template <typename V>
+cudaError_t head_split_as(void* q, void* k, void* v, const void* qkv, int64_t B, int64_t H, int64_t T, int64_t hdv, cudaStream_t stream) {
+    return launch_dependent(head_split_kernel<V>, token_blocks(B * T), 256, stream, static_cast<V*>(q), static_cast<V*>(k),
+                            static_cast<V*>(v), static_cast<const V*>(qkv), B * T, static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv));
+}
 }  // namespace
 
 cudaError_t launch_head_merge(void* y, const void* x, int64_t B, int64_t H, int64_t T, int64_t hd, int elem_bytes,
                               cudaStream_t stream) {
-    if (vec16_ok({y, x}, hd, elem_bytes)) {
-        const int64_t hdv = hd * elem_bytes / 16;
-        head_merge_kernel<uint4><<<static_cast<unsigned>(copy_grid(B * H * T * hdv)), 256, 0, stream>>>(
-            static_cast<uint4*>(y), static_cast<const uint4*>(x), B, H, T, hdv);
-    } else if (elem_bytes == 4) {
-        head_merge_kernel<uint32_t><<<static_cast<unsigned>(copy_grid(B * H * T * hd)), 256, 0, stream>>>(
-            static_cast<uint32_t*>(y), static_cast<const uint32_t*>(x), B, H, T, hd);
-    } else {
-        head_merge_kernel<uint16_t><<<static_cast<unsigned>(copy_grid(B * H * T * hd)), 256, 0, stream>>>(
-            static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), B, H, T, hd);
-    }
-    count_launch(1);
-    return cudaGetLastError();
+    if (vec16_ok({y, x}, hd, elem_bytes)) return head_merge_as<uint4>(y, x, B, H, T, hd * elem_bytes / 16, stream);
+    return elem_bytes == 4 ? head_merge_as<uint32_t>(y, x, B, H, T, hd, stream) : head_merge_as<uint16_t>(y, x, B, H, T, hd, stream);
 }
 
 cudaError_t launch_head_split(void* q, void* k, void* v, const void* qkv, int64_t B, int64_t H, int64_t T, int64_t hd,
                               int elem_bytes, cudaStream_t stream) {
-    if (vec16_ok({q, k, v, qkv}, hd, elem_bytes)) {
-        const int64_t hdv = hd * elem_bytes / 16;
-        head_split_kernel<uint4><<<static_cast<unsigned>(copy_grid(3 * B * H * T * hdv)), 256, 0, stream>>>(
-            static_cast<uint4*>(q), static_cast<uint4*>(k), static_cast<uint4*>(v), static_cast<const uint4*>(qkv), B, H,
-            T, hdv);
-    } else if (elem_bytes == 4) {
-        head_split_kernel<uint32_t><<<static_cast<unsigned>(copy_grid(3 * B * H * T * hd)), 256, 0, stream>>>(
-            static_cast<uint32_t*>(q), static_cast<uint32_t*>(k), static_cast<uint32_t*>(v),
-            static_cast<const uint32_t*>(qkv), B, H, T, hd);
-    } else {
-        head_split_kernel<uint16_t><<<static_cast<unsigned>(copy_grid(3 * B * H * T * hd)), 256, 0, stream>>>(
-            static_cast<uint16_t*>(q), static_cast<uint16_t*>(k), static_cast<uint16_t*>(v),
-            static_cast<const uint16_t*>(qkv), B, H, T, hd);
-    }
-    count_launch(1);
-    return cudaGetLastError();
+    if (vec16_ok({q, k, v, qkv}, hd, elem_bytes)) return head_split_as<uint4>(q, k, v, qkv, B, H, T, hd * elem_bytes / 16, stream);
+    return elem_bytes == 4 ? head_split_as<uint32_t>(q, k, v, qkv, B, H, T, hd, stream)
+                           : head_split_as<uint16_t>(q, k, v, qkv, B, H, T, hd, stream);
 }
+
+namespace {
+template <typename T, bool VEC>
+cudaError_t softmax_as(T* y, const T* x, int64_t rows, int64_t tq, int64_t tk, int causal, cudaStream_t stream) {
+    const unsigned grid = static_cast<unsigned>((rows + 3) / 4);   // four rows per block of four warps
+    if (tk <= 256) return launch_dependent(softmax_rows_kernel<T, 8, VEC>, grid, 128, stream, y, x, rows, tq, tk, causal);
+    if (tk <= 512) return launch_dependent(softmax_rows_kernel<T, 16, VEC>, grid, 128, stream, y, x, rows, tq, tk, causal);
+    if (tk <= 1024) return launch_dependent(softmax_rows_kernel<T, 32, VEC>, grid, 128, stream, y, x, rows, tq, tk, causal);
+    if (tk <= 2048) return launch_dependent(softmax_rows_kernel<T, 64, VEC>, grid, 128, stream, y, x, rows, tq, tk, causal);
+    return launch_dependent(softmax_long_rows_kernel<T>, grid, 128, stream, y, x, rows, tq, tk, causal);
+}
+template <typename T>
+cudaError_t softmax_typed(void* y, const void* x, int64_t rows, int64_t tq, int64_t tk, int causal, cudaStream_t stream) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0 && tk % (16 / static_cast<int64_t>(sizeof(T))) == 0;
+    return vec ? softmax_as<T, true>(static_cast<T*>(y), static_cast<const T*>(x), rows, tq, tk, causal, stream)
+               : softmax_as<T, false>(static_cast<T*>(y), static_cast<const T*>(x), rows, tq, tk, causal, stream);
+}
+}  // namespace
 
 cudaError_t launch_softmax_fwd(void* y, const void* x, int64_t rows, int64_t tq, int64_t tk,
                                int is_bf16, int causal, cudaStream_t stream) {
-    constexpr int kRowsPerBlock = 4;  // one warp per row
-    const unsigned grid = static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock);
-    if (is_bf16)
-        softmax_rows_kernel<__nv_bfloat16><<<grid, kRowsPerBlock * 32, 0, stream>>>(
-            static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(x), rows, tq, tk, causal);
-    else
-        softmax_rows_kernel<float><<<grid, kRowsPerBlock * 32, 0, stream>>>(
-            static_cast<float*>(y), static_cast<const float*>(x), rows, tq, tk, causal);
-    count_launch(1);
-    return cudaGetLastError();
+    return is_bf16 ? softmax_typed<__nv_bfloat16>(y, x, rows, tq, tk, causal, stream)
+                   : softmax_typed<float>(y, x, rows, tq, tk, causal, stream);
 }
 
 cudaError_t launch_softmax_bwd(void* ds, const void* p, const void* dp, int64_t rows, int64_t tk,
                                int is_bf16, cudaStream_t stream) {
-    constexpr int kRowsPerBlock = 4;
+    constexpr int kRowsPerBlock = 4;   // one warp per row
     const unsigned grid = static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock);
     if (is_bf16)
-        softmax_rows_bwd_kernel<__nv_bfloat16><<<grid, kRowsPerBlock * 32, 0, stream>>>(
-            static_cast<__nv_bfloat16*>(ds), static_cast<const __nv_bfloat16*>(p),
-            static_cast<const __nv_bfloat16*>(dp), rows, tk);
-    else
-        softmax_rows_bwd_kernel<float><<<grid, kRowsPerBlock * 32, 0, stream>>>(
-            static_cast<float*>(ds), static_cast<const float*>(p), static_cast<const float*>(dp),
-            rows, tk);
-    count_launch(1);
-    return cudaGetLastError();
+        return launch_dependent(softmax_rows_bwd_kernel<__nv_bfloat16>, grid, kRowsPerBlock * 32, stream, static_cast<__nv_bfloat16*>(ds),
+                                static_cast<const __nv_bfloat16*>(p), static_cast<const __nv_bfloat16*>(dp), rows, tk);
+    return launch_dependent(softmax_rows_bwd_kernel<float>, grid, kRowsPerBlock * 32, stream, static_cast<float*>(ds),
+                            static_cast<const float*>(p), static_cast<const float*>(dp), rows, tk);
 }
 
 }  // namespace llmt_b200

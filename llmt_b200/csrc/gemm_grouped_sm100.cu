@@ -63,19 +63,18 @@ constexpr int kEpilogueWarps = 8;
 constexpr int kProducerHelperWarp = 10;  // first of the helper TMA producer warps (CTA pairs only)
 constexpr int kProducerHelpers = 1;
 constexpr int kSideWarp = 11;            // works on the exchange that rides along, nothing else
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8;
 constexpr int kRing = 4;                             // scheduler ring entries
 constexpr uint32_t kATileBytes = BM * BK * 2;        // 16 KB
 constexpr uint32_t kStoreBufBytes = 32 * 128;        // one staging buffer: 32 rows x 128 bytes
-// Per CTA and stage: the A tile plus room for the widest B tile.  A CTA pair (CG = 2)
-// splits B between its two CTAs, so a stage is smaller: six of them fit where a single CTA
-// has four.  The main loop is bound by the bytes in flight: a stage is refilled about 1.7 us
-// after its MMAs retire (commit -> producer -> TMA -> L2 -> shared memory -> MMA issuer), and a
-// pair consumes 32 KB per CTA every 0.3 us, so anything below ~180 KB of stages starves the
-// tensor pipe (measured with five stages: 0.34-0.43 us per k-block).
-#ifndef LLMT_B200_PAIR_STAGES
-#define LLMT_B200_PAIR_STAGES 6
-#endif
+// Operand stages.  A stage holds the A tile and this CTA's share of the B tile (a CTA pair, CG = 2, splits B
+// between its two CTAs), sized for the widest tile of the launch, and the launch has as many as fit kStageRegion:
+// 6 for a pair's 256-wide tiles, 8 for its 128-wide ones; 4 for a single CTA's 256-wide tiles, 8 for its 64-wide
+// ones.  The main loop is bound by the latency of a stage's round trip (commit -> producer -> TMA -> L2 -> shared
+// memory -> MMA issuer: about 1.7 us) divided by the number of stages: with 256-wide pairs and five
+// stages 0.34-0.43 us per k-block instead of 0.33, with four stages for every width of a single CTA 0.36 us
+// for a 64-wide tile's k-block as for a 256-wide one's.
+constexpr uint32_t kStageRegion = 192 * 1024;
 // 16-byte sums one lane of a side warp keeps in flight.  More is slower, not faster: at 16 the
 // exchange's requests crowd the GEMM's own loads out of the memory system (two GPUs, GPT-2 step:
 // 0.427 ms at 8, 0.435 at 4, 0.453 at 16, 0.550 at 32).
@@ -86,13 +85,10 @@ constexpr uint32_t kStoreBufBytes = 32 * 128;        // one staging buffer: 32 r
 #define LLMT_B200_PAIR_STORE_BUFS 1
 #endif
 template <int CG> struct Geo {
-    static constexpr uint32_t kBRegionBytes = (256 / CG) * BK * 2;
-    static constexpr uint32_t kStageBytes = kATileBytes + kBRegionBytes;
-    static constexpr int kStages = CG == 2 ? LLMT_B200_PAIR_STAGES : 4;
     static constexpr int kStoreBufs = CG == 2 ? LLMT_B200_PAIR_STORE_BUFS : 1;   // staging buffers per epilogue warp
     static constexpr uint32_t kStagingBytes = kEpilogueWarps * kStoreBufs * kStoreBufBytes;
     static constexpr uint32_t kScalarBytes = kMaxGroupProblems * static_cast<uint32_t>(sizeof(ProblemScalars));
-    static constexpr uint32_t kSmemBytes = 1024 /* control block + alignment */ + kStages * kStageBytes + kStagingBytes + kScalarBytes;
+    static constexpr uint32_t kSmemBytes = 1024 /* control block + alignment */ + kStageRegion + kStagingBytes + kScalarBytes;
 };
 static_assert(Geo<1>::kSmemBytes <= 227 * 1024 && Geo<2>::kSmemBytes <= 227 * 1024, "shared-memory budget");
 constexpr uint32_t kBlock64Bytes = 64 * BK * 2;      // one 64-wide MN-major block
@@ -511,8 +507,6 @@ template <uint32_t V> struct Sig { static constexpr uint32_t value = V; };
 
 template <int CG, bool kLse>
 __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
-    constexpr int kStages = Geo<CG>::kStages;
-    constexpr uint32_t kStageBytes = Geo<CG>::kStageBytes;
     constexpr int kStoreBufs = Geo<CG>::kStoreBufs;
     constexpr bool kPair = CG == 2;
     constexpr int kTileRows = BM * CG;  // rows of C one scheduled tile covers
@@ -528,7 +522,9 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
     // stages and the epilogue warps' staging buffers.
     Control* ctl = reinterpret_cast<Control*>(smem_raw);
     const uint32_t smem_base = (smem_u32(smem_raw) + static_cast<uint32_t>(sizeof(Control)) + 1023u) & ~1023u;
-    const uint32_t staging_base = smem_base + kStages * kStageBytes;
+    const uint32_t staging_base = smem_base + kStageRegion;
+    const int n_stages = gp.stages;
+    const uint32_t stage_bytes = gp.stage_bytes;
     // The problems' scalars, copied from the kernel parameters (see ProblemScalars).
     ProblemScalars* sp = reinterpret_cast<ProblemScalars*>(smem_raw + (staging_base - smem_u32(smem_raw)) + Geo<CG>::kStagingBytes);
     volatile int* abort_flag = &ctl->abort_flag;
@@ -538,7 +534,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(smem_u32(&ctl->full[s]), 1);
             // A stage is released by the MMAs that read it (one commit) and by the eight epilogue
             // warps, which read it too when the tile sums its A operand for a bias gradient; for
@@ -653,7 +649,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
         const int n_turns = kPair ? 1 + kProducerHelpers : 1;
         const int my_turn = warp == 0 ? 0 : warp - kProducerHelperWarp + 1;
         int turn = 0;      // whose k-block `seq` is: producers take them round robin, across tiles
-        uint32_t seq = 0;  // k-blocks streamed so far by this CTA; k-block `seq` uses stage seq % kStages
+        uint32_t seq = 0;  // k-blocks streamed so far by this CTA; k-block `seq` uses stage seq % n_stages
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -799,7 +795,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                     // the arming arrival).
                     if (my_map != nullptr) {
                         const int k0 = kb * BK;
-                        const uint32_t dst = smem_base + static_cast<uint32_t>(stage) * kStageBytes + my_off;
+                        const uint32_t dst = smem_base + static_cast<uint32_t>(stage) * stage_bytes + my_off;
                         const int x = my_x + (k_is_x ? k0 : 0), y = my_y + (k_is_y ? k0 : 0);
                         if (kPair) tma_load_4d_pair(dst, my_map, on_leader(&ctl->full[stage]), x, y, tc.bz, tc.bw);
                         else tma_load_4d(dst, my_map, smem_u32(&ctl->full[stage]), x, y, tc.bz, tc.bw);
@@ -812,7 +808,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                     }
                 }
                 if (++turn == n_turns) turn = 0;
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                if (++stage == n_stages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -850,7 +846,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                                              kDevWaitSmemFull, stage, wait_ns);
                     if (!ok) break;
                     tc_fence_after_thread_sync();
-                    const uint32_t stage_off = static_cast<uint32_t>(stage) * (kStageBytes >> 4);
+                    const uint32_t stage_off = static_cast<uint32_t>(stage) * (stage_bytes >> 4);
                     const uint32_t a_lo = a_lo_base + stage_off;
                     const uint32_t b_lo = b_lo_base + stage_off;
 #pragma unroll
@@ -862,7 +858,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                         umma_bf16_cg<CG>(d_tmem, da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
                     }
                     umma_commit_cg<CG>(smem_u32(&ctl->empty[stage]));  // frees the stage when the MMAs retire
-                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    if (++stage == n_stages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
                 umma_commit_cg<CG>(smem_u32(&ctl->tmem_full[acc]));
@@ -1018,7 +1014,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                     if (!ok) break;
                     landed_bits ^= 1u << e_stage;
-                    const uint32_t base = smem_base + static_cast<uint32_t>(e_stage) * kStageBytes + blk + half8;
+                    const uint32_t base = smem_base + static_cast<uint32_t>(e_stage) * stage_bytes + blk + half8;
 #pragma unroll
                     for (int r = 0; r < 8; ++r) {
                         const uint32_t row = static_cast<uint32_t>(8 * ew + r);
@@ -1032,7 +1028,7 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&ctl->empty[e_stage]));  // this warp is done with the stage
-                    if (++e_stage == kStages) { e_stage = 0; e_phase ^= 1u; }
+                    if (++e_stage == n_stages) { e_stage = 0; e_phase ^= 1u; }
                 }
                 if (!ok) break;
                 // The eight warps' sums meet in the staging buffers (free once the TMA stores that
@@ -1081,8 +1077,9 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                 sum_phase ^= 1u;
             } else {
                 const int total = e_stage + nkb;
-                e_phase ^= static_cast<uint32_t>(total / kStages) & 1u;
-                e_stage = total % kStages;
+                const int rounds = static_cast<int>(div_by(static_cast<uint32_t>(total), static_cast<uint32_t>(n_stages), gp.inv_stages));
+                e_phase ^= static_cast<uint32_t>(rounds) & 1u;
+                e_stage = total - rounds * n_stages;
             }
             // Everything a step needs is read from the problem's scalars ONCE per tile, into
             // registers: a step is a chain of dependent instructions executed by a warp that has
@@ -1565,7 +1562,11 @@ size_t tc_grouped_smem_bytes() {
     return Geo<1>::kSmemBytes > Geo<2>::kSmemBytes ? Geo<1>::kSmemBytes : Geo<2>::kSmemBytes;
 }
 
-int tc_pair_stages() { return Geo<2>::kStages; }
+uint32_t tc_stage_bytes(bool pairs, int bn) { return kATileBytes + static_cast<uint32_t>(bn / (pairs ? 2 : 1)) * (BK * 2); }
+int tc_stages(bool pairs, int bn) {
+    const int n = static_cast<int>(kStageRegion / tc_stage_bytes(pairs, bn));
+    return n < kMaxStages ? n : kMaxStages;
+}
 int tc_dbias_rows_per_cta() { return kDbiasRowsPerCta; }
 int tc_dbias_finish_per_cta() { return kDbiasFinishPerCta; }
 
