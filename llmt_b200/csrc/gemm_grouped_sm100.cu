@@ -158,6 +158,39 @@ __device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, vola
 }
 
 
+// The same for a converged warp: every lane polls, so the warp stays converged and what it issues next may be
+// issued by any of its lanes.
+__device__ __forceinline__ bool bounded_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, DeviceStatus* st, int code,
+                                                  int detail, uint64_t limit_ns) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    uint64_t t0 = 0;
+    uint32_t spins = 0;
+    for (;;) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if ((++spins & 255u) == 0u) {
+            int stop = 0;
+            if ((threadIdx.x & 31) == 0) {
+                if (*abort_flag) {
+                    stop = 1;
+                } else {
+                    const uint64_t now = globaltimer_ns();
+                    if (t0 == 0) {
+                        t0 = now;
+                    } else if (now - t0 > limit_ns) {
+                        if (atomicCAS(&st->code, 0, code) == 0) {
+                            st->detail = detail;
+                            st->block = static_cast<int32_t>(blockIdx.x);
+                        }
+                        *abort_flag = 1;
+                        stop = 1;
+                    }
+                }
+            }
+            if (__shfl_sync(0xffffffffu, stop, 0) != 0) return false;
+        }
+    }
+}
+
 // n / d with the reciprocal of d at hand.  One thread of the MMA warp decodes a ticket between
 // two tiles, where a hardware-emulated integer division (a long dependent chain) is exposed:
 // below 2^24 the float product is within one of the quotient and two compares fix it.
@@ -639,18 +672,19 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
         // that is issued late is a bubble in the tensor pipe later: a producer must be waiting at
         // a stage's barrier when the stage frees.  One iteration costs a few hundred cycles of
         // barrier and issue latency, which a single warp cannot hide (a third warp measured no
-        // further gain).  In each warp the whole warp walks the loop; lane 0 does the barrier
-        // bookkeeping and lane L issues the L-th box of a stage, so the up to six TMA boxes of a k-block
-        // (MN-major operands come in 64-wide blocks) leave in one issue slot.  Warp 0 of the
-        // leader also runs the scheduler.
+        // further gain).  The whole warp walks the loop with warp-uniform values and one elected lane
+        // issues a stage's boxes (one for a K-major operand, one per 64-wide block of an MN-major one): the TMA
+        // instruction takes its operands from uniform registers, so boxes issued by different lanes are
+        // issued one after the other anyway, each after its own moves into them (260 cycles per k-block of a
+        // producer warp, which is what a single CTA's k-block took).  Warp 0 of the leader also runs the
+        // scheduler.
         const bool scheduler = warp == 0 && leader;
         // A single CTA streams 48 KB per k-block and is bound by that, not by issue latency:
         // there the helper stays idle and warp 0 takes every k-block.
         const int n_turns = kPair ? 1 + kProducerHelpers : 1;
         const int my_turn = warp == 0 ? 0 : warp - kProducerHelperWarp + 1;
-        int turn = 0;      // whose k-block `seq` is: producers take them round robin, across tiles
-        uint32_t seq = 0;  // k-blocks streamed so far by this CTA; k-block `seq` uses stage seq % n_stages
-        int stage = 0;
+        int turn = 0;      // whose k-block is next: producers take them round robin, across tiles
+        int stage = 0;     // k-blocks use the stages in turn, across tiles
         uint32_t phase = 0;
         bool ok = true;
         // A ticket is drawn when the producer is nearly ready to stream that tile: a few k-blocks
@@ -703,109 +737,111 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
                 for (int q = 0; q < 3; ++q) st_async_cluster_v4(dst + 16u * q, w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3], bar);
             }
         };
+        const uint32_t full0 = kPair ? mapa_shared(smem_u32(&ctl->full[0]), 0u) : smem_u32(&ctl->full[0]);   // (the leader's)
         for (int it = 0; ok; ++it) {
             const int slot = it % kRing;
             const uint32_t sphase = static_cast<uint32_t>(it / kRing) & 1u;
-            if (lane == 0) {
-                if (scheduler && early) {
-                    early = false;
-                } else if (scheduler) {
-                    ok = bounded_wait<kPair>(smem_u32(&ctl->sched_empty[slot]), sphase ^ 1u, abort_flag, status,
-                                             kDevWaitSched, slot, wait_ns);
-                    if (ok) {
-                        const int raw = it == 0 ? first_ticket
-                                      : !dynamic ? prev_ticket + n_sched
-                                      : next_ticket != kNotDrawn ? next_ticket : atomicAdd(gp.sched_counter, 1) + n_sched;
-                        next_ticket = kNotDrawn;
-                        publish(slot, raw);
+            if (scheduler) {
+                if (lane == 0) {
+                    if (early) {
+                        early = false;
+                    } else {
+                        ok = bounded_wait<kPair>(smem_u32(&ctl->sched_empty[slot]), sphase ^ 1u, abort_flag, status,
+                                                 kDevWaitSched, slot, wait_ns);
+                        if (ok) {
+                            const int raw = it == 0 ? first_ticket
+                                          : !dynamic ? prev_ticket + n_sched
+                                          : next_ticket != kNotDrawn ? next_ticket : atomicAdd(gp.sched_counter, 1) + n_sched;
+                            next_ticket = kNotDrawn;
+                            publish(slot, raw);
+                        }
                     }
-                } else {
-                    // In the peer CTA warp 0 arms the ring barrier for the leader's stores.
-                    if (kPair && warp == 0)
-                        mbar_arrive_expect_tx(smem_u32(&ctl->sched_full[slot]), static_cast<uint32_t>(sizeof(TileCoord)));
-                    ok = bounded_wait<kPair>(smem_u32(&ctl->sched_full[slot]), sphase, abort_flag, status,
-                                             kDevWaitSched, 48 + slot, wait_ns);
                 }
+                __syncwarp();  // lane 0's ring write is visible to the warp
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            } else {
+                // In the peer CTA warp 0 arms the ring barrier for the leader's stores.
+                if (kPair && warp == 0 && lane == 0)
+                    mbar_arrive_expect_tx(smem_u32(&ctl->sched_full[slot]), static_cast<uint32_t>(sizeof(TileCoord)));
+                __syncwarp();
+                ok = bounded_wait_warp(smem_u32(&ctl->sched_full[slot]), sphase, abort_flag, status, kDevWaitSched, 48 + slot, wait_ns);
             }
-            __syncwarp();  // lane 0's ring write is visible to the warp
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             const TileCoord tc = ctl->ring[slot];
             __syncwarp();
             if (!scheduler && lane == 0) release_ring_slot(slot);
-            const int t = tc.t;
+            const int t = uniform(tc.t);
             if (t < 0) break;
             if (t < gp.colsum_total || t >= gp.fin_begin) continue;  // a dbias ticket: work for the epilogue warps only
-            const ProblemScalars& p = sp[tc.prob];
-            const GroupProblem& pm = gp.prob[tc.prob];  // for the addresses of its tensor maps only
-            const int bn = p.bn, a_mn = p.a_mn, b_mn = p.b_mn;
+            const int prob = uniform(tc.prob);
+            const ProblemScalars& p = sp[prob];
+            const GroupProblem& pm = gp.prob[prob];  // for the addresses of its tensor maps only
+            const int bn = uniform(p.bn);
+            const bool a_mn = uniform(p.a_mn) != 0, b_mn = uniform(p.b_mn) != 0;
             const int bn_cta = bn / CG;                         // B columns this CTA stages
-            const int m0 = tc.m_tile * kTileRows + static_cast<int>(rank) * BM;
-            const int n0 = tc.n_tile * bn + static_cast<int>(rank) * bn_cta;
+            const int m0 = uniform(tc.m_tile) * kTileRows + static_cast<int>(rank) * BM;
+            const int n0 = uniform(tc.n_tile) * bn + static_cast<int>(rank) * bn_cta;
+            const int kb0 = uniform(tc.kb0), kb1 = uniform(tc.kb1), bz = uniform(tc.bz), bw = uniform(tc.bw);
             const uint32_t tx = kATileBytes + static_cast<uint32_t>(bn_cta) * (BK * 2);
-            // This lane's box: destination offset inside the stage, tensor map, and the
-            // coordinates (the k coordinate advances with the k-block).
-            const int n_a = a_mn ? 2 : 1, n_b = b_mn ? (bn_cta >> 6) : 1;
-            const CUtensorMap* my_map = nullptr;
-            uint32_t my_off = 0;
-            int my_x = 0, my_y = 0;
-            bool k_is_x = false, k_is_y = false;
-            if (lane < n_a) {
-                my_map = &pm.map_a;
-                if (a_mn) { my_off = lane * kBlock64Bytes; my_x = m0 + 64 * lane; k_is_y = true; }
-                else      { my_y = m0; k_is_x = true; }
-            } else if (lane < n_a + n_b) {
-                const int j = lane - n_a;
-                my_map = &pm.map_b;
-                my_off = kATileBytes;
-                if (b_mn) { my_off += j * kBlock64Bytes; my_x = n0 + 64 * j; k_is_y = true; }
-                else      { my_y = n0; k_is_x = true; }
-            }
+            const int n_b = bn_cta >> 6;                        // 64-wide blocks of an MN-major B
+            auto load_box = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+                if (kPair) tma_load_4d_pair(dst, map, bar, x, y, bz, bw);
+                else tma_load_4d(dst, map, bar, x, y, bz, bw);
+            };
             if (!dep_waited) {   // the first loads are next: the previous kernel must be done
                 grid_dependency_wait();
                 dep_waited = true;
             }
-            const bool tile_sums = p.dbias_mode == 3 && tc.n_tile == 0;  // the epilogue warps read this tile's A stages
-            const int draw_kb = tc.kb1 - kDrawAhead > tc.kb0 ? tc.kb1 - kDrawAhead : tc.kb0;
-            const int publish_kb = tc.kb1 - tc.kb0 >= kMinEarlyKblocks ? tc.kb1 - kPublishAhead : 0x7fffffff;
+            const bool tile_sums = uniform(p.dbias_mode == 3 && tc.n_tile == 0 ? 1 : 0) != 0;  // the epilogue warps read this tile's A stages
+            const int draw_kb = kb1 - kDrawAhead > kb0 ? kb1 - kDrawAhead : kb0;
+            const int publish_kb = kb1 - kb0 >= kMinEarlyKblocks ? kb1 - kPublishAhead : 0x7fffffff;
             const int after_own = n_turns > 1 ? 1 : 0;
-            for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++seq) {
-                if (kb >= draw_kb && scheduler && lane == 0) {  // (the first test is warp-uniform and false on most k-blocks)
-                    if (dynamic && kb == draw_kb) next_ticket = atomicAdd(gp.sched_counter, 1) + n_sched;
-                    if (kb >= publish_kb && !early && turn == after_own) {
-                        const int nslot = (it + 1) % kRing;
-                        const uint32_t nphase = static_cast<uint32_t>((it + 1) / kRing) & 1u;
-                        // one poll: a ring that is still full is waited for at the top
-                        if (mbar_try_wait(smem_u32(&ctl->sched_empty[nslot]), nphase ^ 1u)) {
-                            publish(nslot, dynamic ? next_ticket : prev_ticket + n_sched);
-                            next_ticket = kNotDrawn;
-                            early = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (scheduler && kb >= draw_kb) {  // (false on most k-blocks)
+                    if (lane == 0) {
+                        if (dynamic && kb == draw_kb) next_ticket = atomicAdd(gp.sched_counter, 1) + n_sched;
+                        if (kb >= publish_kb && !early && turn == after_own) {
+                            const int nslot = (it + 1) % kRing;
+                            const uint32_t nphase = static_cast<uint32_t>((it + 1) / kRing) & 1u;
+                            // one poll: a ring that is still full is waited for at the top
+                            if (mbar_try_wait(smem_u32(&ctl->sched_empty[nslot]), nphase ^ 1u)) {
+                                publish(nslot, dynamic ? next_ticket : prev_ticket + n_sched);
+                                next_ticket = kNotDrawn;
+                                early = true;
+                            }
                         }
                     }
+                    __syncwarp();
                 }
                 if (turn == my_turn) {
-                    if (lane == 0)
-                        ok = bounded_wait<kPair>(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, status,
-                                                 kDevWaitSmemEmpty, stage, wait_ns);
-                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    ok = bounded_wait_warp(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, status, kDevWaitSmemEmpty, stage, wait_ns);
                     if (!ok) break;
                     // The loads leave first: the latency from "stage free" to "load issued" is part of
                     // every stage's cycle.  The bookkeeping follows; bytes that land before the
                     // barrier is armed are counted all the same (the phase cannot complete without
                     // the arming arrival).
-                    if (my_map != nullptr) {
+                    if (elect_one()) {
                         const int k0 = kb * BK;
-                        const uint32_t dst = smem_base + static_cast<uint32_t>(stage) * stage_bytes + my_off;
-                        const int x = my_x + (k_is_x ? k0 : 0), y = my_y + (k_is_y ? k0 : 0);
-                        if (kPair) tma_load_4d_pair(dst, my_map, on_leader(&ctl->full[stage]), x, y, tc.bz, tc.bw);
-                        else tma_load_4d(dst, my_map, smem_u32(&ctl->full[stage]), x, y, tc.bz, tc.bw);
-                    }
-                    if (lane == 0) {
+                        const uint32_t a_dst = smem_base + static_cast<uint32_t>(stage) * stage_bytes, b_dst = a_dst + kATileBytes;
+                        const uint32_t bar = full0 + 8u * static_cast<uint32_t>(stage);
+                        if (a_mn) {
+                            load_box(a_dst, &pm.map_a, bar, m0, k0);
+                            load_box(a_dst + kBlock64Bytes, &pm.map_a, bar, m0 + 64, k0);
+                        } else {
+                            load_box(a_dst, &pm.map_a, bar, k0, m0);
+                        }
+                        if (b_mn) {
+                            for (int j = 0; j < n_b; ++j)
+                                load_box(b_dst + static_cast<uint32_t>(j) * kBlock64Bytes, &pm.map_b, bar, n0 + 64 * j, k0);
+                        } else {
+                            load_box(b_dst, &pm.map_b, bar, k0, n0);
+                        }
                         // The leader's barrier counts the bytes of both CTAs of a pair.
                         if (leader) mbar_arrive_expect_tx(smem_u32(&ctl->full[stage]), tx * CG);
                         // the stage's next release: nobody but the MMAs will read it
                         if (!tile_sums) mbar_arrive_count(smem_u32(&ctl->empty[stage]), kEpilogueWarps);
                     }
+                    __syncwarp();
                 }
                 if (++turn == n_turns) turn = 0;
                 if (++stage == n_stages) { stage = 0; phase ^= 1u; }
@@ -813,55 +849,62 @@ __device__ __forceinline__ void tc_grouped_body(const GroupParams& gp) {
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0 && leader) {
+        // The whole warp walks the loop with warp-uniform values; one elected lane, always the same, issues the
+        // MMAs and the commits.  (With one lane in the loop the descriptors were ordinary registers that had to be
+        // moved into uniform ones for every MMA: 250 cycles per k-block for the four of them.)
+        if (leader) {
             constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
             int stage = 0;
             uint32_t phase = 0;
             // Accumulator slot q lives in TMEM buffer q & 1 and is on its (q >> 1)-th use.
             uint32_t acc_seq = 0;
             bool ok = true;
+            const uint32_t tmem0 = uniform(tmem_base);
             for (int it = 0; ok; ++it) {
                 const int slot = it % kRing;
                 const uint32_t sphase = static_cast<uint32_t>(it / kRing) & 1u;
-                ok = bounded_wait(smem_u32(&ctl->sched_full[slot]), sphase, abort_flag, status,
-                                  kDevWaitSched, 16 + slot, wait_ns);
+                ok = bounded_wait_warp(smem_u32(&ctl->sched_full[slot]), sphase, abort_flag, status, kDevWaitSched, 16 + slot, wait_ns);
                 if (!ok) break;
                 const int4 head = *reinterpret_cast<const int4*>(&ctl->ring[slot]);  // t, prob, kb0, kb1
-                release_ring_slot(slot);
-                const int t = head.x;
+                __syncwarp();
+                if (lane == 0) release_ring_slot(slot);
+                const int t = uniform(head.x);
                 if (t < 0) break;
                 if (t < gp.colsum_total || t >= gp.fin_begin) continue;
-                const int nkb = head.w - head.z;
+                const int nkb = uniform(head.w - head.z);
                 const uint4 mc = ctl->mma_consts[head.y];
-                const uint32_t idesc = mc.x, a_lo_base = mc.y, b_lo_base = mc.z;
-                const uint32_t step_a = mc.w & 0xFFFFu, step_b = mc.w >> 16;
+                const uint32_t idesc = uniform(mc.x), a_lo_base = uniform(mc.y), b_lo_base = uniform(mc.z);
+                const uint32_t steps = uniform(mc.w);
+                const uint32_t step_a = steps & 0xFFFFu, step_b = steps >> 16;
                 const int acc = static_cast<int>(acc_seq & 1u);
-                ok = bounded_wait<kPair>(smem_u32(&ctl->tmem_empty[acc]), ((acc_seq >> 1) & 1u) ^ 1u, abort_flag,
-                                         status, kDevWaitTmemEmpty, acc, wait_ns);
+                ok = bounded_wait_warp(smem_u32(&ctl->tmem_empty[acc]), ((acc_seq >> 1) & 1u) ^ 1u, abort_flag, status, kDevWaitTmemEmpty,
+                                       acc, wait_ns);
                 if (!ok) break;
                 tc_fence_after_thread_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc) * kAccStride;
+                const uint32_t d_tmem = tmem0 + static_cast<uint32_t>(acc) * kAccStride;
                 for (int i = 0; i < nkb; ++i) {
-                    ok = bounded_wait<kPair>(smem_u32(&ctl->full[stage]), phase, abort_flag, status,
-                                             kDevWaitSmemFull, stage, wait_ns);
+                    ok = bounded_wait_warp(smem_u32(&ctl->full[stage]), phase, abort_flag, status, kDevWaitSmemFull, stage, wait_ns);
                     if (!ok) break;
                     tc_fence_after_thread_sync();
-                    const uint32_t stage_off = static_cast<uint32_t>(stage) * (stage_bytes >> 4);
-                    const uint32_t a_lo = a_lo_base + stage_off;
-                    const uint32_t b_lo = b_lo_base + stage_off;
+                    if (elect_one()) {
+                        const uint32_t stage_off = static_cast<uint32_t>(stage) * (stage_bytes >> 4);
+                        const uint32_t a_lo = a_lo_base + stage_off;
+                        const uint32_t b_lo = b_lo_base + stage_off;
 #pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                        const uint64_t da = (static_cast<uint64_t>(kDescHi) << 32) |
-                                            static_cast<uint64_t>(a_lo + kk * step_a);
-                        const uint64_t db = (static_cast<uint64_t>(kDescHi) << 32) |
-                                            static_cast<uint64_t>(b_lo + kk * step_b);
-                        umma_bf16_cg<CG>(d_tmem, da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                            const uint64_t da = (static_cast<uint64_t>(kDescHi) << 32) |
+                                                static_cast<uint64_t>(a_lo + kk * step_a);
+                            const uint64_t db = (static_cast<uint64_t>(kDescHi) << 32) |
+                                                static_cast<uint64_t>(b_lo + kk * step_b);
+                            umma_bf16_cg<CG>(d_tmem, da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        umma_commit_cg<CG>(smem_u32(&ctl->empty[stage]));  // frees the stage when the MMAs retire
+                        if (i + 1 == nkb) umma_commit_cg<CG>(smem_u32(&ctl->tmem_full[acc]));
                     }
-                    umma_commit_cg<CG>(smem_u32(&ctl->empty[stage]));  // frees the stage when the MMAs retire
+                    __syncwarp();
                     if (++stage == n_stages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                umma_commit_cg<CG>(smem_u32(&ctl->tmem_full[acc]));
                 ++acc_seq;
             }
         }

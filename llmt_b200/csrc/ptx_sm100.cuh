@@ -105,6 +105,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// One lane of a converged warp, the same one every time (true in that lane).  An instruction behind it is issued once
+// per warp with its operands in uniform registers, as the TMA and tcgen05 instructions take them.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(is));
+    return is != 0;
+}
+// A value that is the same in every lane, as the compiler can see it.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // --------------------------------------------------------------------- TMA --
 
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
