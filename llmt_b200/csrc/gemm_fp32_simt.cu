@@ -583,7 +583,8 @@ repack_bf16_kernel(const __grid_constant__ RepackJobs jobs) {
         } else {
             src[i] = src[0] + i * dc;
             dst[i] = dst[0] + i * dc;
-            left[i] = left[0] - i * dc;
+            // (a unit that starts at the end of the padded row belongs to the next row)
+            left[i] = c0 + i * dc < p.ld_dst ? left[0] - i * dc : -8;
         }
         lo[i] = hi[i] = make_uint4(0, 0, 0, 0);
         if (left[i] >= 8) {

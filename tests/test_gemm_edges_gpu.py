@@ -285,3 +285,27 @@ def test_attention_products_on_the_packed_qkv_layout(dt):
     assert oracle.rel_fro(scores[b_, h_].float().cpu().numpy(), p_ref) <= 2 * tol
     o_ref = oracle.gemm(scores[b_, h_].float().cpu().numpy(), vh)
     assert oracle.rel_fro(y[b_, :, h_ * hd:(h_ + 1) * hd].float().cpu().numpy(), o_ref) <= tol
+
+
+@pytest.mark.parametrize("cols", [2041, 2050, 4095, 5650, 8193])
+def test_repacked_copy_of_long_rows_stays_within_them(cols):
+    """Rows of more than 2048 columns whose padded pitch ends inside the copying block's reach: every row of the
+    copy is the source's row and zeros up to the padded pitch, and nothing behind the last one is touched (16 rows:
+    the copy fills its 256-byte rounded share of the workspace to the last byte)."""
+    rows, pitch = 16, (cols + 7) // 8 * 8
+    a = _bf16_dev(np.random.default_rng(cols).standard_normal((rows, cols)))
+    b = _bf16_dev(np.random.default_rng(7).standard_normal((16, cols)) * 0.1)
+    c = torch.zeros(rows, 16, device=DEV)
+    d = L.make_desc(c, a, b, False, True, splits=1)
+    need = L.workspace_bytes(d, a, b)
+    assert need == 2 * rows * pitch * 2
+    ws = torch.full((need + 256,), 0x5A, dtype=torch.uint8, device=DEV)
+    d.workspace, d.workspace_bytes = ws.data_ptr(), need
+    for _ in range(10):
+        ws[:need] = 0x5A
+        L.gemm_desc(d, c, a, b)
+        copies = ws[:need].view(torch.bfloat16).view(2, rows, pitch)
+        for x, y in ((a, copies[0]), (b, copies[1])):
+            assert torch.equal(x, y[:, :cols]) and bool((y[:, cols:] == 0).all())
+        assert bool((ws[need:] == 0x5A).all())
+    assert oracle.rel_fro(c.cpu().numpy(), oracle.gemm(a.float().cpu().numpy(), b.float().cpu().numpy(), False, True)) <= TOL
