@@ -20,8 +20,8 @@ OBJ_DIR = os.path.join(HERE, "_build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libllmt_b200.so")
 
-SOURCES = ["capi.cu", "gemm_grouped_sm100.cu", "gemm_fp32_simt.cu", "grad_allreduce_sm100.cu", "cross_entropy.cu"]
-HEADERS = ["common.h", "ptx_sm100.cuh", os.path.join("..", "..", "include", "llmt_b200.h")]
+SOURCES = ["capi.cu", "gemm_grouped_sm100.cu", "gemm_fp32_simt.cu", "gemm_fp32_sm100.cu", "grad_allreduce_sm100.cu", "cross_entropy.cu"]
+HEADERS = ["common.h", "ptx_sm100.cuh", "waits_sm100.cuh", "gemm_fp32.cuh", os.path.join("..", "..", "include", "llmt_b200.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -921,6 +921,9 @@ int run_fp32(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b
     if (d->batch > 65535) return fail(LLMT_B200_ERR_UNSUPPORTED, "matmul: fp32 path supports batch <= 65535");
     p.dbias = d->dbias;
     p.dbias_beta = d->dbias_beta;
+    p.wait_limit_ns = g_wait_limit_ns;
+    p.status = device_status_ptr();
+    if (p.status == nullptr) return fail(LLMT_B200_ERR_CUDA, "cannot resolve the device status word");
     const cudaError_t e = launch_fp32_gemm(p, stream);
     if (e != cudaSuccess) return fail(LLMT_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     return LLMT_B200_OK;

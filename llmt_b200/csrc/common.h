@@ -202,6 +202,8 @@ struct Fp32GemmParams {
     int32_t tiles_m, tiles_n, splits;
     int64_t k_per_split;
     int32_t vec_a, vec_b, vec_c;
+    DeviceStatus* status;       // (the tensor-core form's bounded waits)
+    uint64_t wait_limit_ns;
 };
 
 // Copies of operands that TMA cannot address, one launch for all of a call's (see repack_bf16_kernel).
@@ -298,6 +300,10 @@ int tc_stages(bool pairs, int bn);             // and how many of them a CTA has
 int tc_dbias_rows_per_cta(void);
 int tc_dbias_finish_per_cta(void);
 cudaError_t launch_fp32_gemm(const Fp32GemmParams& p, cudaStream_t stream);
+// The tensor-core form (gemm_fp32_sm100.cu): its tiling of a problem and estimated cycles (bn 0: not for it); the launch.
+struct Fp32TcPlan { int bn, splits; int64_t cost; };
+Fp32TcPlan fp32_tc_plan(const Fp32GemmParams& p);
+cudaError_t launch_fp32_tc(const Fp32GemmParams& p, const Fp32TcPlan& plan, cudaStream_t stream);
 cudaError_t launch_zero_f32(float* dst, int64_t n, cudaStream_t stream);
 cudaError_t launch_repack_bf16(RepackJobs jobs, cudaStream_t stream);
 cudaError_t launch_softmax_fwd(void* y, const void* x, int64_t rows, int64_t tq, int64_t tk,

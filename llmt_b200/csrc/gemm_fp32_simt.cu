@@ -1,15 +1,17 @@
-// Strict-fp32 GEMM (fp32 storage, fp32 FMA arithmetic, no tensor cores) and the element-wise and
+// fp32 GEMM (fp32 storage, fp32 FMA arithmetic, no tensor cores) and the element-wise and
 // row-wise kernels around the GEMMs.
 //
 // The fp32 path must agree with llmt's fp32 golden tensors at rtol 1e-5 (llmt runs cuBLASLt with
 // CUBLAS_COMPUTE_32F and refuses TF32, src/kernels/matmul.cpp:33-36,72-77); tcgen05 has no
-// full-precision fp32 MMA, so it runs on the CUDA cores.  k ascends inside a split and the splits
-// are added in order: the sum order is fixed, results are bitwise reproducible.
+// full-precision fp32 MMA, so this kernel runs on the CUDA cores.  k ascends inside a split and the splits
+// are added in order: the sum order is fixed, results are bitwise reproducible.  Problems that fill tiles of 128 rows
+// go to the tensor cores in three bf16 parts instead (gemm_fp32_sm100.cu; the rule is in launch_fp32_gemm).
 #include <cuda_bf16.h>
 
 #include <initializer_list>
 
 #include "common.h"
+#include "gemm_fp32.cuh"
 
 namespace llmt_b200 {
 
@@ -151,30 +153,6 @@ __device__ __forceinline__ void f32_load_stage(uint32_t dst, const float* __rest
             }
         }
     }
-}
-
-__device__ __forceinline__ float4 ld_dsmem16(uint32_t addr, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float ld_dsmem4(uint32_t addr, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-
-__device__ __forceinline__ float f32_finish(const Fp32GemmParams& p, float acc, const float* dst, int64_t col) {
-    float v = p.alpha * acc;
-    if (p.beta != 0.0f) v += p.beta * *dst;
-    if (p.epi_flags & kEpiBias)
-        v += p.bias_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]) : static_cast<const float*>(p.bias)[col];
-    if (p.epi_flags & kEpiGelu) v = gelu_tanh_precise(v);
-    return v;
 }
 
 // Grid: x = tiles * splits (the `splits` CTAs of a cluster share one tile), z = batch item.
@@ -799,6 +777,12 @@ cudaError_t launch_fp32_gemm(const Fp32GemmParams& in, cudaStream_t stream) {
             }
         }
     }
+    const Fp32TcPlan tc = fp32_tc_plan(in);
+    // The tensor-core form where its model says so: both models count cycles and are pure functions of the sizes.  With few
+    // rows or a short reduction a tile of 128 rows and its start cost more than the FMAs save (32 x 768 x 768: 8.6 us here,
+    // 11.1 us there; 1000 x 100 x 100: 7.4 and 8.9), everything larger gains (256 x 256 x 64, 48 times: 17.7 and 15.2;
+    // 256 x 2304 x 768: 36 and 16; 4096^3: 2780 and 830).
+    if (tc.bn != 0 && tc.cost < best) return launch_fp32_tc(in, tc, stream);
     return form == 0 ? launch_fp32_size<2, 2, 1>(p, stream) : form == 1 ? launch_fp32_size<1, 2, 2>(p, stream) : launch_fp32_size<1, 2, 4>(p, stream);
 }
 
