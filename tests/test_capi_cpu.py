@@ -411,3 +411,11 @@ def test_aux_epilogues_are_never_split_along_k():
     assert "splits=1" in L.plan(d)
     d.plan_splits = 4
     assert "splits=1" in L.plan(d)
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 2304, 768), (128, 2304, 768), (512, 2304, 768), (1024, 768, 768), (2048, 768, 3072)])
+def test_bf16_results_are_split_only_where_a_second_launch_pays(m, n, k):
+    d = _desc(m=m, n=n, k=k, lda=k, ldb=k, ldc=n, dtype_c=L.BF16)
+    assert "splits=1 " in L.plan(d) and L.workspace_bytes(d) == 0
+    d.dtype_c = L.FP32                            # an fp32 result keeps its parts: fewer would be less exact
+    assert "splits=1 " not in L.plan(d) and L.workspace_bytes(d) > 0
