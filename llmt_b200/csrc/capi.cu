@@ -178,15 +178,12 @@ int choose_splits(int64_t tiles, int kblocks_total, int sms) {
     return splits;
 }
 
-// Cycles that splitting a reduction adds: a second launch that waits for the first one's last store (about 4.5 us with its
-// own start and end) and the partial sums on their way to memory and back.
-int64_t split_cost(int64_t partial_bytes) { return 8500 + partial_bytes / 2000; }
-
-// The most parts a reduction is split into: what fills the machine, by a model of waves of equal tiles that leans towards
-// splitting.  It bounds the workspace that a problem may ask for.  An fp32 result keeps to it: the tensor core's
-// additions truncate and parts are added rounded to nearest, so fewer parts would be less exact (768 x 768 x 2048:
-// 2.1e-6 whole, 1.0e-6 in two parts, 0.5e-6 in four).  A bf16 result takes fewer where that is faster.
-int most_splits(int64_t m, int64_t n, int64_t k, int64_t batch, int units, int force_bn, bool pairs, bool b_mn, int epi_step, bool c_bf16) {
+// The parts a reduction is split into: what fills the machine, by a model of waves of equal tiles that leans towards
+// splitting.  The tensor core's additions truncate and parts are added rounded to nearest, so the number of parts is a
+// matter of precision as well as of speed (768 x 768 x 2048, sums before any rounding of the result: 2.1e-6 whole, 1.0e-6
+// in two parts, 0.5e-6 in four), for a bf16 result as for an fp32 one.  Hence it follows from the problem alone, and only
+// the tiles' width is chosen by measured costs: the sums' bits do not depend on it.
+int reduction_parts(int64_t m, int64_t n, int64_t k, int64_t batch, int units, int force_bn, bool pairs, bool b_mn, int epi_step, bool c_bf16) {
     const int kblocks_total = ceil_div(k, 64);
     const int64_t tiles_m = ceil_div(m, pairs ? 256 : 128);
     int64_t best_cost = 0;
@@ -229,49 +226,40 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int dbias_mode,
     const int cands[4] = {256, 192, 128, 64};
     const int tiles_m = ceil_div(m, pairs ? 256 : 128);
     const int kblocks_total = ceil_div(k, 64);
-    int best_bn = 0, best_splits = 1;
+    int best_bn = 0;
     int64_t best_cost = 0;
-    const int most = force_splits > 0 ? force_splits : most_splits(m, n, k, batch, sms, force_bn, pairs, b_mn, epi_step, c_bf16);
+    const int parts = force_splits > 0 ? force_splits : reduction_parts(m, n, k, batch, sms, force_bn, pairs, b_mn, epi_step, c_bf16);
+    const int splits = parts <= kblocks_total ? parts : kblocks_total > 0 ? kblocks_total : 1;
+    const int kps = ceil_div(kblocks_total, splits);
     for (int bn : cands) {
         if (force_bn != 0 && bn != force_bn) continue;
         if (pairs && (bn == 64 || (b_mn && bn % 128 != 0))) continue;
         // Never pick a tile wider than needed when a narrower one covers n in one column.
         if (force_bn == 0 && bn > 64 && n <= bn - 64 && !(pairs && bn == 128)) continue;
         const int64_t tiles = static_cast<int64_t>(tiles_m) * ceil_div(n, bn) * batch;
-        // 1, 2, 3, 4, 6, 8, 24 and the most
-        auto next = [&](int w) { const int q = w < 4 ? w + 1 : w < 8 ? w + 2 : 3 * w; return w < most && q > most ? most : q; };
-        for (int want = force_splits > 0 || !c_bf16 ? most : 1; want <= most; want = next(want)) {
-            int splits = want;
-            if (splits > kblocks_total) splits = kblocks_total > 0 ? kblocks_total : 1;
-            const int64_t partial = splits > 1 ? static_cast<int64_t>(splits) * batch * m * n * 4 : 0;
-            const int kps = ceil_div(kblocks_total, splits);
-            const int64_t waves = (tiles * splits + sms - 1) / sms;
-            // Estimated cycles: per wave the longer of main loop and epilogue, one pass over the partials when split.  (512 x
-            // 2304 x 768 in two splits: 15.4 us, whole 8.3; 512 x 768 x 3072 whole 15.0, in four 12.9, in eight 14.6.)
-            const int unit_cols = (c_bf16 && splits == 1) ? 64 : 32;
-            const int steps = ((bn / unit_cols + 1) / 2) * (unit_cols / 32);
-            const int64_t main_loop = static_cast<int64_t>(kblock_cost(bn, pairs)) * (kps > 0 ? kps : 1);
-            const int64_t epilogue = static_cast<int64_t>(steps) * (splits == 1 ? epi_step : 1000);
-            int64_t cost = waves * ((main_loop > epilogue ? main_loop : epilogue) + 4 * bn);
-            if (splits > 1) cost += split_cost(partial);
-            if (best_bn == 0 || cost < best_cost) {
-                best_bn = bn;
-                best_cost = cost;
-                best_splits = splits;
-            }
+        const int64_t waves = (tiles * splits + sms - 1) / sms;
+        // Estimated cycles: per wave the longer of main loop and epilogue.
+        const int unit_cols = (c_bf16 && splits == 1) ? 64 : 32;
+        const int steps = ((bn / unit_cols + 1) / 2) * (unit_cols / 32);
+        const int64_t main_loop = static_cast<int64_t>(kblock_cost(bn, pairs)) * (kps > 0 ? kps : 1);
+        const int64_t epilogue = static_cast<int64_t>(steps) * (splits == 1 ? epi_step : 1000);
+        const int64_t cost = waves * ((main_loop > epilogue ? main_loop : epilogue) + 4 * bn);
+        if (best_bn == 0 || cost < best_cost) {
+            best_bn = bn;
+            best_cost = cost;
         }
     }
     TcPlan pl{};
     if (best_bn == 0) best_bn = pairs ? 128 : 64;
-    finish_plan(&pl, m, n, k, batch, dbias_mode, best_bn, best_splits, pairs);
+    finish_plan(&pl, m, n, k, batch, dbias_mode, best_bn, splits, pairs);
     return pl;
 }
 
 // Plan of a problem that shares its launch with others: the queue is dynamic, so wave quantisation of one problem does
-// not matter; the widest tile up to `widest` that wastes nothing, and, where `may_split`, only reductions that are longer
-// than the average load of an SM in parts.
+// not matter; the widest tile up to `widest` that wastes nothing, and only reductions that are longer than the average
+// load of an SM in parts (whatever the tiles' width: see reduction_parts).
 TcPlan make_group_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int dbias_mode, int sms,
-                       int64_t group_kblock_tiles, int force_bn, int force_splits, bool pairs, bool b_mn, int widest, bool may_split) {
+                       int64_t group_kblock_tiles, int force_bn, int force_splits, bool pairs, bool b_mn, int widest) {
     int bn = widest;
     if (n <= 64) bn = pairs ? 128 : 64;
     else if (n <= 128) bn = 128;
@@ -281,7 +269,7 @@ TcPlan make_group_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int dbias
     int splits = 1;
     if (force_splits > 0) {
         splits = force_splits;
-    } else if (may_split) {
+    } else {
         const int64_t avg = group_kblock_tiles / sms;  // k-blocks per SM if perfectly balanced
         const int64_t target = avg > 16 ? avg : 16;
         if (kblocks_total > target + target / 4) splits = ceil_div(kblocks_total, target);
@@ -940,29 +928,25 @@ bool plan_group(const llmt_b200_gemm_desc* descs, int count, TcPlan* plans) {
         plans[0] = plan_single(&descs[0]);
         return plans[0].pairs != 0;
     }
-    // Tile width and splitting for the launch as a whole: the tiles spread over the units, but the last one to start is
-    // waited for, and a split adds a launch per problem.  Many tiles: 256 wide; few: narrower ones that need no splitting.
+    // Tile width for the launch as a whole: the tiles spread over the units, but the last one to start is waited for.  Many
+    // tiles: 256 wide; few: narrower ones.
     int64_t best_cost = 0;
     for (int widest = 256; widest >= 128; widest -= 128) {
-        for (int may_split = 1; may_split >= 0; --may_split) {
-            TcPlan tried[kMaxGroupProblems];
-            int64_t sum = 0, longest = 0, extra = 0;
-            for (int i = 0; i < count; ++i) {
-                const llmt_b200_gemm_desc& d = descs[i];
-                TcPlan& pl = tried[i];
-                pl = make_group_plan(d.m, d.n, d.k, d.batch, dbias_mode_of(&d), sms, work, d.plan_tile_n, splits_wanted(&d), pairs, d.trans_b == 0,
-                                     widest, may_split != 0 || d.dtype_c != LLMT_B200_BF16);   // (an fp32 result: see most_splits)
-                const int64_t tile = static_cast<int64_t>(kblock_cost(pl.bn, pairs)) * pl.kblocks_per_split + 4 * pl.bn + 1500;
-                sum += tile * pl.num_tiles;
-                if (tile > longest) longest = tile;
-                if (pl.splits > 1) extra += split_cost(static_cast<int64_t>(pl.splits) * d.m * d.n * (d.batch > 0 ? d.batch : 1) * 4);
-            }
-            const int64_t spread = sum / sms + longest / 3;
-            const int64_t cost = (spread > longest ? spread : longest) + extra;
-            if (best_cost == 0 || cost < best_cost) {
-                best_cost = cost;
-                for (int i = 0; i < count; ++i) plans[i] = tried[i];
-            }
+        TcPlan tried[kMaxGroupProblems];
+        int64_t sum = 0, longest = 0;
+        for (int i = 0; i < count; ++i) {
+            const llmt_b200_gemm_desc& d = descs[i];
+            TcPlan& pl = tried[i];
+            pl = make_group_plan(d.m, d.n, d.k, d.batch, dbias_mode_of(&d), sms, work, d.plan_tile_n, splits_wanted(&d), pairs, d.trans_b == 0, widest);
+            const int64_t tile = static_cast<int64_t>(kblock_cost(pl.bn, pairs)) * pl.kblocks_per_split + 4 * pl.bn + 1500;
+            sum += tile * pl.num_tiles;
+            if (tile > longest) longest = tile;
+        }
+        const int64_t spread = sum / sms + longest / 3;
+        const int64_t cost = spread > longest ? spread : longest;
+        if (best_cost == 0 || cost < best_cost) {
+            best_cost = cost;
+            for (int i = 0; i < count; ++i) plans[i] = tried[i];
         }
     }
     return pairs;

@@ -414,8 +414,22 @@ def test_aux_epilogues_are_never_split_along_k():
 
 
 @pytest.mark.parametrize("m,n,k", [(8, 2304, 768), (128, 2304, 768), (512, 2304, 768), (1024, 768, 768), (2048, 768, 3072)])
-def test_bf16_results_are_split_only_where_a_second_launch_pays(m, n, k):
+def test_bf16_results_are_summed_in_as_many_parts_as_fp32_ones(m, n, k):
+    # the tensor core's additions truncate, parts are added rounded to nearest: fewer parts would be less exact
     d = _desc(m=m, n=n, k=k, lda=k, ldb=k, ldc=n, dtype_c=L.BF16)
-    assert "splits=1 " in L.plan(d) and L.workspace_bytes(d) == 0
-    d.dtype_c = L.FP32                            # an fp32 result keeps its parts: fewer would be less exact
-    assert "splits=1 " not in L.plan(d) and L.workspace_bytes(d) > 0
+    parts = int(re.search(r"splits=(\d+) ", L.plan(d)).group(1))
+    assert parts > 1 and L.workspace_bytes(d) > 0
+    d.dtype_c = L.FP32
+    assert f"splits={parts} " in L.plan(d)
+
+
+@pytest.mark.parametrize("m,i,o", [(512, 768, 2304), (512, 768, 3072), (1537, 771, 1283), (128, 768, 3072)])
+def test_a_grouped_bf16_result_keeps_its_parts(m, i, o):
+    # dX [m, i] = dY [m, o] W [o, i] beside the layer's dW, as bf16 and as fp32: the same scratch for the same parts
+    def dx_bytes(code):
+        dx = _desc(m=m, n=i, k=o, lda=o + o % 2, ldb=i + i % 2, ldc=i, trans_b=0, dtype_c=code)
+        dw = _desc(m=o, n=i, k=m, trans_a=1, trans_b=0, lda=o + o % 2, ldb=i + i % 2, ldc=i, dtype_c=L.FP32, beta=1.0)
+        out = (ctypes.c_uint64 * 2)()
+        assert L.lib().llmt_b200_gemm_grouped_workspace_bytes((L.GemmDesc * 2)(dx, dw), 2, out) == L.OK
+        return out[0]
+    assert dx_bytes(L.BF16) == dx_bytes(L.FP32) > m * i * 4
