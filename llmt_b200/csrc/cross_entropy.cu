@@ -49,16 +49,17 @@ __device__ __forceinline__ void lse_warp_combine(float& m, float& s) {
 }
 
 // The (maximum, sum of exponentials) pair of the x[0 .. v) that thread `tid` of `nt` sees: 16-byte loads, four in flight.
-// EXP: the exponential (expf, or __expf where the caller's accuracy allows).
+// EXP: the exponential (expf, or __expf where the caller's accuracy allows).  A -inf adds nothing wherever it stands, also
+// where it is all that the thread has seen yet (no difference of two infinities is formed).
 template <typename EXP>
 __device__ __forceinline__ void lse_of_row(const float* x, int64_t v, int tid, int nt, EXP ex, float& m, float& s) {
     m = -INFINITY;
     s = 0.0f;
     auto take = [&](float xi) {
         if (xi > m) {
-            s = s * ex(m - xi) + 1.0f;  // exp(-inf) = 0 covers the first element
+            s = s * ex(m - xi) + 1.0f;  // exp(-inf) = 0 covers the first finite element
             m = xi;
-        } else {
+        } else if (xi != -INFINITY) {
             s += ex(xi - m);
         }
     };
@@ -68,7 +69,8 @@ __device__ __forceinline__ void lse_of_row(const float* x, int64_t v, int tid, i
             s *= ex(m - mx);
             m = mx;
         }
-        s += (ex(q.x - m) + ex(q.y - m)) + (ex(q.z - m) + ex(q.w - m));
+        const float from = m == -INFINITY ? 0.0f : m;
+        s += (ex(q.x - from) + ex(q.y - from)) + (ex(q.z - from) + ex(q.w - from));
     };
     int64_t head = static_cast<int64_t>((16u - (reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / 4;
     if (head > v) head = v;
@@ -85,6 +87,7 @@ __device__ __forceinline__ void lse_of_row(const float* x, int64_t v, int tid, i
     }
     for (; i < n4; i += nt) take4(x4[i]);
     for (int64_t j = head + 4 * n4 + tid; j < v; j += nt) take(x[j]);
+    if (m == -INFINITY && s != 0.0f) m = 0.0f;   // nothing but NaN and -inf: not an empty set, the NaN stays
 }
 
 // The pairs of W warps into every one of their threads, in a fixed order.  `sh`: 2 * 32 floats of the block (W > 1).

@@ -135,6 +135,48 @@ def test_cross_entropy_bwd_against_the_oracle(rows, vocab, in_place):
     assert_close(out.cpu().numpy(), want, rtol=5e-5, atol=1e-7, what="dlogits")
 
 
+@pytest.mark.parametrize("rows,vocab", [(5, 128), (9, 1000), (4, 2048), (9, 4096), (5, 50257), (200, 16387)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_cross_entropy_with_banned_tokens(rows, vocab, offset):
+    """Logits of -inf (banned tokens, padding columns of the vocabulary) add nothing, wherever their runs lie: one warp, eight
+    and 32 per row, rows on and off a 16-byte boundary, forward and backward, against numpy in 64 bits.  A run of NaN
+    makes the row's loss NaN."""
+    rng = np.random.default_rng(rows * 5 + vocab)
+    x = (rng.standard_normal((rows, vocab)) * 3.0).astype(np.float32)
+    runs = [(0, 40), (vocab // 2 // 4 * 4, 12), (100, 8), (vocab - 40, 40), (0, 0)]
+    for r in range(rows):
+        lo, n = runs[r % len(runs)]
+        x[r, lo:lo + n] = -np.inf
+    if rows > 5:
+        x[5], x[5, 0] = -np.inf, 1.0          # one token left
+    t = np.array([rng.choice(np.flatnonzero(np.isfinite(x[r]))) for r in range(rows)], dtype=np.int32)
+    w = rng.random(rows).astype(np.float32) + 0.1
+    pitch = vocab + 3 - (vocab + 3) % 4 + offset
+    xd = torch.zeros(rows, pitch, device=DEV)[:, offset:offset + vocab]
+    xd.copy_(torch.from_numpy(x))
+    td, wd = torch.from_numpy(t).to(DEV), torch.from_numpy(w).to(DEV)
+    loss, nll = _ce(xd, td, wd)
+    x64 = x.astype(np.float64)
+    top = x64.max(axis=1, keepdims=True)
+    lse = np.log(np.exp(x64 - top).sum(axis=1, keepdims=True)) + top
+    want = w * (lse[:, 0] - x64[np.arange(rows), t])
+    assert_close(nll, want, rtol=1e-5, atol=1e-5, what="row_nll")
+    assert_close(loss, np.array([want.sum() / w.astype(np.float64).sum()]), rtol=1e-5, atol=1e-6, what="loss")
+    grad = np.exp(x64 - lse)
+    grad[np.arange(rows), t] -= 1.0
+    grad *= (w.astype(np.float64) / w.astype(np.float64).sum())[:, None]
+    apart = torch.full((rows, vocab), float("nan"), device=DEV)
+    L.cross_entropy_bwd(apart, xd, td, wd)
+    L.cross_entropy_bwd(xd, xd, td, wd)
+    for got in (apart, xd):
+        assert_close(got.cpu().numpy(), grad, rtol=5e-5, atol=1e-7, what="dlogits")
+        assert bool((got[torch.from_numpy(np.isneginf(x)).to(DEV)] == 0.0).all())
+    xd.copy_(torch.from_numpy(x))
+    xd[rows - 1, 64:96] = float("nan")
+    loss, nll = _ce(xd, td, wd)
+    assert np.isnan(nll[rows - 1]) and np.isfinite(nll[:rows - 1]).all() and np.isnan(loss).all()
+
+
 @pytest.mark.parametrize("m,vocab,k,out_dtype,reuse", [(256, 512, 128, torch.bfloat16, True), (300, 1000, 192, torch.float32, False),
                                                        (1024, 50257, 768, torch.bfloat16, True)])
 def test_lm_head_dlogits_from_the_product(m, vocab, k, out_dtype, reuse):
