@@ -425,21 +425,24 @@ softmax_rows_kernel(T* y, const T* x, int64_t rows, int64_t tq, int64_t tk, int 
     for (int i = 0; i < N / kPer; ++i) {
         const int c = (i * 32 + lane) * kPer;
         if (c >= tk) break;
-        const float* from = v + i * kPer;
+        float* from = v + i * kPer;
+        // (zeros by themselves, not as exp(-inf) * scale: in a row with a NaN or an infinity the scale is NaN)
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) from[j] = c + j < live ? from[j] * scale : 0.0f;
         if (VEC) {
             uint32_t q[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (sizeof(T) == 4) {
-                    q[j] = __float_as_uint(from[j] * scale);
+                    q[j] = __float_as_uint(from[j]);
                 } else {
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(from[(2 * j) % kPer] * scale, from[(2 * j + 1) % kPer] * scale);
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(from[(2 * j) % kPer], from[(2 * j + 1) % kPer]);
                     q[j] = *reinterpret_cast<const uint32_t*>(&h);
                 }
             }
             *reinterpret_cast<uint4*>(out + c) = make_uint4(q[0], q[1], q[2], q[3]);
         } else {
-            Elem<T>::put(out, c, from[0] * scale);
+            Elem<T>::put(out, c, from[0]);
         }
     }
 }
