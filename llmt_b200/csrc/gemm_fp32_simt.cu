@@ -88,7 +88,7 @@ __device__ __forceinline__ uint64_t dup2(float v) {
 // One operand's share of a stage: ROWS rows (the m or n index, from r0) x DEPTH, zero beyond
 // `rows` and beyond `kend`.  KC: stored with k contiguous.
 template <bool KC, int ROWS, int DEPTH, int THREADS>
-__device__ __forceinline__ void f32_load_stage(uint32_t dst, const float* __restrict__ x, int64_t ld, int64_t r0, int64_t rows,
+__device__ __forceinline__ void f32_load_stage(uint32_t dst, const float* x, int64_t ld, int64_t r0, int64_t rows,
                                                int64_t k0, int64_t kend, bool vec) {
     const int tid = threadIdx.x;
     const bool inside = r0 + ROWS <= rows && k0 + DEPTH <= kend;   // the whole stage exists: no test per element
@@ -571,8 +571,8 @@ repack_bf16_kernel(const __grid_constant__ RepackJobs jobs) {
         if (left[i] >= 8) {
             const uintptr_t at = reinterpret_cast<uintptr_t>(src[i]);
             const uint4* w = reinterpret_cast<const uint4*>(at & ~static_cast<uintptr_t>(15));
-            lo[i] = __ldg(w);
-            if ((at & 15u) != 0 && (last_lane || left[i] < 16)) hi[i] = __ldg(w + 1);
+            lo[i] = *w;
+            if ((at & 15u) != 0 && (last_lane || left[i] < 16)) hi[i] = w[1];
         } else if (left[i] > 0) {
             lo[i] = repack_tail(src[i], left[i]);
         }
@@ -598,7 +598,7 @@ repack_bf16_kernel(const __grid_constant__ RepackJobs jobs) {
 //   split: out[part][b, h, t, d] = qkv[b, t, part*A + h*hd + d],  A = H*hd, part = 0..parts-1
 template <typename V>
 __global__ void __launch_bounds__(256)
-head_merge_kernel(V* __restrict__ y, const V* __restrict__ x, int64_t tokens, uint32_t H, int64_t T, uint32_t hdv) {
+head_merge_kernel(V* __restrict__ y, const V* x, int64_t tokens, uint32_t H, int64_t T, uint32_t hdv) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t width = H * hdv;
     for (int64_t token = blockIdx.x; token < tokens; token += gridDim.x) {
@@ -612,7 +612,7 @@ head_merge_kernel(V* __restrict__ y, const V* __restrict__ x, int64_t tokens, ui
 
 template <typename V>
 __global__ void __launch_bounds__(256)
-head_split_kernel(V* __restrict__ q, V* __restrict__ k, V* __restrict__ v, const V* __restrict__ qkv, int64_t tokens, uint32_t H, int64_t T,
+head_split_kernel(V* __restrict__ q, V* __restrict__ k, V* __restrict__ v, const V* qkv, int64_t tokens, uint32_t H, int64_t T,
                   uint32_t hdv) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t width = H * hdv;

@@ -110,6 +110,8 @@ __device__ __forceinline__ void tile_at(const Fp32GemmParams& p, int64_t t, Tile
     o->b = p.b + bi * p.stride_b + bo * p.stride_b_outer;
 }
 
+// (Plain loads: the operands are still being written by the kernel before while this one's blocks are resident, which the
+// read-only path does not allow.)
 // One operand's W rows (the m or n index) x 64 of a k-block are W / 16 groups of four values a thread, each four that
 // neighbour each other in memory.  K-major: group u is row 16 u + tid / 16, k 4 (tid % 16).  MN: k-row 8 u + tid / 32
 // (W = 128) or 16 u + tid / 16, rows 4 (tid % (W / 4)).  Rows beyond the matrix repeat its last ones (their results
@@ -119,7 +121,7 @@ __device__ __forceinline__ LoadForm load_form(int64_t k0, int64_t kend, bool vec
     return k0 + kBK > kend ? kLoadEdge : vec ? kLoadVec : kLoadScalar;
 }
 template <bool MN, int W>
-__device__ __forceinline__ float4 load_group(int u, LoadForm form, const float* __restrict__ x, int64_t ld, int64_t r0, int64_t rows, int64_t k0,
+__device__ __forceinline__ float4 load_group(int u, LoadForm form, const float* x, int64_t ld, int64_t r0, int64_t rows, int64_t k0,
                                              int64_t kend) {
     constexpr int kLanes = MN ? W / 4 : 16, kStep = kSplitThreads / kLanes;
     const int tid = threadIdx.x;
@@ -128,21 +130,20 @@ __device__ __forceinline__ float4 load_group(int u, LoadForm form, const float* 
         const int64_t row = r0 + across < rows ? r0 + across : rows - 1;
         const int64_t k = k0 + along;
         const float* s = x + row * ld + k;
-        if (form == kLoadVec) return __ldg(reinterpret_cast<const float4*>(s));
-        if (form == kLoadScalar) return make_float4(__ldg(s), __ldg(s + 1), __ldg(s + 2), __ldg(s + 3));
-        return make_float4(k < kend ? __ldg(s) : 0.0f, k + 1 < kend ? __ldg(s + 1) : 0.0f, k + 2 < kend ? __ldg(s + 2) : 0.0f,
-                           k + 3 < kend ? __ldg(s + 3) : 0.0f);
+        if (form == kLoadVec) return *reinterpret_cast<const float4*>(s);
+        if (form == kLoadScalar) return make_float4(s[0], s[1], s[2], s[3]);
+        return make_float4(k < kend ? s[0] : 0.0f, k + 1 < kend ? s[1] : 0.0f, k + 2 < kend ? s[2] : 0.0f,
+                           k + 3 < kend ? s[3] : 0.0f);
     }
     const int64_t c = r0 + along;
     const float* s = x + (k0 + across) * ld;
-    if (form == kLoadVec) return __ldg(reinterpret_cast<const float4*>(s + (c < rows ? c : rows - 4)));   // (rows is a multiple of 4)
+    if (form == kLoadVec) return *reinterpret_cast<const float4*>(s + (c < rows ? c : rows - 4));   // (rows is a multiple of 4)
     if (form == kLoadEdge && k0 + across >= kend) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int64_t end = rows - 1;
-    return make_float4(__ldg(s + (c < end ? c : end)), __ldg(s + (c + 1 < end ? c + 1 : end)), __ldg(s + (c + 2 < end ? c + 2 : end)),
-                       __ldg(s + (c + 3 < end ? c + 3 : end)));
+    return make_float4(s[c < end ? c : end], s[c + 1 < end ? c + 1 : end], s[c + 2 < end ? c + 2 : end], s[c + 3 < end ? c + 3 : end]);
 }
 template <bool MN, int W>
-__device__ __forceinline__ void load_operand(float4 (&v)[W / 16], LoadForm form, const float* __restrict__ x, int64_t ld, int64_t r0,
+__device__ __forceinline__ void load_operand(float4 (&v)[W / 16], LoadForm form, const float* x, int64_t ld, int64_t r0,
                                              int64_t rows, int64_t k0, int64_t kend) {
 #pragma unroll
     for (int u = 0; u < W / 16; ++u) v[u] = load_group<MN, W>(u, form, x, ld, r0, rows, k0, kend);
@@ -183,7 +184,7 @@ __device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst
 // registers are free and has until the same group's turn a whole block later.
 template <bool MN, int W, bool SUMS>
 __device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst, float& amax, bool sums, float4& sum, bool more,
-                                               const float* __restrict__ x, int64_t ld, int64_t r0, int64_t rows, int64_t k0, int64_t kend,
+                                               const float* x, int64_t ld, int64_t r0, int64_t rows, int64_t k0, int64_t kend,
                                                bool vec) {
     auto pass = [&](auto form_c) {
         constexpr int kForm = decltype(form_c)::value;
@@ -426,11 +427,11 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
                         for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
 #pragma unroll 1
                         for (int64_t k = kbeg; k < kend; ++k) {
-                            const float av = __ldg(a);
+                            const float av = *a;
                             const float* bj = b;
 #pragma unroll
                             for (int j = 0; j < kCols; ++j) {
-                                acc[j] = fmaf(av, __ldg(bj), acc[j]);
+                                acc[j] = fmaf(av, *bj, acc[j]);
                                 if (n0 + j + 1 < p.n) bj += b_col;   // (columns beyond the matrix repeat its last one)
                             }
                             a += a_step;

@@ -237,10 +237,11 @@ __device__ __forceinline__ void store_chunk_f32(float* dst, const float* v, int 
     }
 }
 
-// 16 bytes of an operand that this kernel only reads.
+// 16 bytes of an operand that is read once.  (Not by the read-only path: the kernel before may still write it while this one's
+// blocks are resident.)
 __device__ __forceinline__ uint4 ld_operand16(const void* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
