@@ -26,10 +26,12 @@
 // 1.0e-7), 512 x 50257 x 768 856 -> 310 (5.0e-7 -> 1.0e-7), dX of that layer 962 -> 400 (1.4e-6 -> 2.7e-7), its dW
 // 824 -> 383 (4.0e-7 -> 9.6e-8), 4096^3 2780 -> 830 (166 TFLOP/s).
 //
-// Values the split cannot carry: an infinity or NaN (its rest is NaN), a finite value whose hi part overflows, and
-// operands so small that the parts or their products leave the normal range.  The first two make the accumulators
-// non-finite, the last shows in the largest magnitudes, which the splitting warps keep: in all of them the warp
-// that owns the sums forms them again with plain fp32 FMAs from the operands as they are.
+// Range: both operands are multiplied by 2^24 before they are split and the sums by 2^-48 afterwards, both exact.  The last
+// bit of any fp32 value, subnormal ones too, is then at 2^-125 or above, so every part is a normal number, and what
+// the accumulators lose below 2^-126 is below 2^-174 of the sums: less than the last bit of the smallest fp32 number, row by
+// row, whatever else a tile holds.  Values the split cannot carry lie at the other end: an infinity or NaN (its
+// rest is NaN), a finite value above 2^103 (it overflows) and sums that pass 2^79.  They all make the accumulators
+// non-finite, and the warp that owns the sums forms them again with plain fp32 FMAs from the operands as they are.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -74,8 +76,7 @@ template <int BN> struct TcGeo {
 struct __align__(16) TcControl {
     uint64_t full[kOpStages], empty[kOpStages];
     uint64_t acc_full[2], acc_empty[2];
-    uint64_t done[kDoneSlots];                            // a tile's operands are all split: amax (and dsums) hold its values
-    float2 amax[kDoneSlots][kSplitWarps];                 // largest magnitudes (A, B)
+    uint64_t done[kDoneSlots];                            // a tile's operands are all split: dsums hold its values (with a fused dbias)
     float dsum[kBM];                                      // a split's share of the fused dbias, for the cluster's addition
     uint32_t tmem_base;
     int abort_flag;
@@ -150,18 +151,50 @@ __device__ __forceinline__ void load_operand(float4 (&v)[W / 16], LoadForm form,
 }
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
-__device__ __forceinline__ float rest_lo(float x, uint32_t h) { return x - __uint_as_float(h << 16); }
-__device__ __forceinline__ float rest_hi(float x, uint32_t h) { return x - __uint_as_float(h & 0xFFFF0000u); }
+__device__ __forceinline__ float low_of(uint32_t h) { return __uint_as_float(h << 16); }
+__device__ __forceinline__ float high_of(uint32_t h) { return __uint_as_float(h & 0xFFFF0000u); }
+// The same on pairs of floats.
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t round2(uint64_t x) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
+    return pack2(lo, hi);
+}
+__device__ __forceinline__ uint64_t negated2(uint32_t h) { return pair2(-low_of(h), -high_of(h)); }
 __device__ __forceinline__ void st_shared8(uint32_t at, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
 }
 
-// Splits a group of four and leaves its parts in their places (128-byte swizzle).
+constexpr float kUp = 0x1p24f, kDown = 0x1p-48f;   // see the range above
+
+// Splits a group of four and leaves its parts in their places (128-byte swizzle).  PACKED: the arithmetic on pairs, taken
+// for K-major operands.  The bits are the same; measured, us, one value at a time and in pairs: 512 x 50257 x 768 with
+// both operands K-major 306 and 294, 4096^3 with both MN-major 952 and 1045.
 template <bool MN, int W>
-__device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst, float& amax) {
+__device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst) {
+    constexpr bool PACKED = !MN;
     constexpr uint32_t kPart = W * kBK * 2;
     constexpr uint32_t kLanes = MN ? W / 4 : 16;
     constexpr uint32_t kStep = kSplitThreads / kLanes;     // 8 or 16 rows of 128 bytes
@@ -170,11 +203,25 @@ __device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst
     const uint32_t blk = MN ? ((tid % kLanes) >> 4) * (64u * 128u) : 0u;
     // (row & 7 is the same for all of a thread's groups)
     const uint32_t at = dst + blk + row * 128u + (((c >> 1) ^ (row & 7u)) << 4) + (c & 1u) * 8u + static_cast<uint32_t>(u) * (kStep * 128u);
-    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-    const uint32_t h0 = pack2(x.x, x.y), h1 = pack2(x.z, x.w);
-    const float r0 = rest_lo(x.x, h0), r1 = rest_hi(x.y, h0), r2 = rest_lo(x.z, h1), r3 = rest_hi(x.w, h1);
-    const uint32_t m0 = pack2(r0, r1), m1 = pack2(r2, r3);
-    const uint32_t l0 = pack2(rest_lo(r0, m0), rest_hi(r1, m0)), l1 = pack2(rest_lo(r2, m1), rest_hi(r3, m1));
+    uint32_t h0, h1, m0, m1, l0, l1;
+    if (PACKED) {
+        const uint64_t up = pair2(kUp, kUp), x0 = pair2(x.x, x.y), x1 = pair2(x.z, x.w);
+        h0 = round2(mul2(x0, up));
+        h1 = round2(mul2(x1, up));
+        const uint64_t r0 = fma2(x0, up, negated2(h0)), r1 = fma2(x1, up, negated2(h1));
+        m0 = round2(r0);
+        m1 = round2(r1);
+        l0 = round2(add2(r0, negated2(m0)));
+        l1 = round2(add2(r1, negated2(m1)));
+    } else {
+        h0 = pack2(x.x * kUp, x.y * kUp);
+        h1 = pack2(x.z * kUp, x.w * kUp);
+        const float r0 = fmaf(x.x, kUp, -low_of(h0)), r1 = fmaf(x.y, kUp, -high_of(h0)), r2 = fmaf(x.z, kUp, -low_of(h1)), r3 = fmaf(x.w, kUp, -high_of(h1));
+        m0 = pack2(r0, r1);
+        m1 = pack2(r2, r3);
+        l0 = pack2(r0 - low_of(m0), r1 - high_of(m0));
+        l1 = pack2(r2 - low_of(m1), r3 - high_of(m1));
+    }
     st_shared8(at, h0, h1);
     st_shared8(at + kPart, m0, m1);
     st_shared8(at + 2 * kPart, l0, l1);
@@ -183,7 +230,7 @@ __device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst
 // Splits the operand's share in hand and loads the next block's, group by group: a group's load is issued as soon as its
 // registers are free and has until the same group's turn a whole block later.
 template <bool MN, int W, bool SUMS>
-__device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst, float& amax, bool sums, float4& sum, bool more,
+__device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst, bool sums, float4& sum, bool more,
                                                const float* x, int64_t ld, int64_t r0, int64_t rows, int64_t k0, int64_t kend,
                                                bool vec) {
     auto pass = [&](auto form_c) {
@@ -191,7 +238,7 @@ __device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst
 #pragma unroll
         for (int u = 0; u < W / 16; ++u) {
             if (SUMS && sums) { sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w; }
-            split_group<MN, W>(u, v[u], dst, amax);
+            split_group<MN, W>(u, v[u], dst);
             if (kForm >= 0) v[u] = load_group<MN, W>(u, static_cast<LoadForm>(kForm), x, ld, r0, rows, k0, kend);
         }
     };
@@ -259,13 +306,13 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
         tile_at(p, t0, &at);
         int kb = 0;
         uint32_t stage = 0, phase = 0, seq = 0;
-        float amax_a = 0.0f, amax_b = 0.0f;
         float4 dsum = make_float4(0.0f, 0.0f, 0.0f, 0.0f), unused = dsum;
         bool sums = AM && p.dbias != nullptr && at.n_tile == 0;
         int64_t m0 = static_cast<int64_t>(at.m_tile) * kBM, n0 = static_cast<int64_t>(at.n_tile) * BN;
         load_operand<AM, kBM>(va, load_form(kbeg, kend, p.vec_a != 0), at.a, p.lda, m0, p.m, kbeg, kend);
         load_operand<BMn, BN>(vb, load_form(kbeg, kend, p.vec_b != 0), at.b, p.ldb, n0, p.n, kbeg, kend);
         bool more = true;
+#pragma unroll 1
         while (more) {
             const bool last = kb + 1 == nk;
             kb = last ? 0 : kb + 1;
@@ -278,29 +325,22 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
             const int64_t k0 = kbeg + static_cast<int64_t>(kb) * kBK;
             if (!bounded_wait_warp(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, p.status, kDevWaitSmemEmpty, 128 + stage, wait_ns)) break;
             const uint32_t dst = stages + stage * G::kStageBytes;
-            split_and_load<AM, kBM, AM>(va, dst, amax_a, sums, dsum, more, at.a, p.lda, m0, p.m, k0, kend, p.vec_a != 0);
-            split_and_load<BMn, BN, false>(vb, dst + 3 * kPartA, amax_b, false, unused, more, at.b, p.ldb, n0, p.n, k0, kend, p.vec_b != 0);
+            split_and_load<AM, kBM, AM>(va, dst, sums, dsum, more, at.a, p.lda, m0, p.m, k0, kend, p.vec_a != 0);
+            split_and_load<BMn, BN, false>(vb, dst + 3 * kPartA, false, unused, more, at.b, p.ldb, n0, p.n, k0, kend, p.vec_b != 0);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctl->full[stage]));
             stage ^= 1u;
             if (stage == 0) phase ^= 1u;
             if (!last) continue;
-            // the tile's largest magnitudes and bias-gradient parts, for the warps that sum
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                amax_a = fmaxf(amax_a, __shfl_xor_sync(0xffffffffu, amax_a, o));
-                amax_b = fmaxf(amax_b, __shfl_xor_sync(0xffffffffu, amax_b, o));
-            }
+            // the tile's bias-gradient parts, for the warps that sum
             if (AM && sums) {   // this warp's k-rows (w, w + 8, ...) of the tile's 128 columns
                 reinterpret_cast<float4*>(dsums + ((seq % kDoneSlots) * kSplitWarps + warp) * kBM)[lane] = dsum;
                 dsum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            if (lane == 0) ctl->amax[seq % kDoneSlots][warp] = make_float2(amax_a, amax_b);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctl->done[seq % kDoneSlots]));
             ++seq;
-            amax_a = amax_b = 0.0f;
             sums = AM && p.dbias != nullptr && at.n_tile == 0;
         }
         grid_launch_dependents();
@@ -385,21 +425,11 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
                     }
                 }
                 if (i + 1 == nk) {
-                    // (before the last release: the splitting warps stay within kDoneSlots tiles)
+                    // (before the last release: the splitting warps stay within kDoneSlots tiles; on every tile, bias gradient or
+                    // not: the code that the compiler makes without it is 5 to 20 % slower)
                     ok = bounded_wait_warp(smem_u32(&ctl->done[seq % kDoneSlots]), (seq / kDoneSlots) & 1u, abort_flag, p.status, kDevWaitSmemFull,
                                            160, wait_ns);
                     if (!ok) break;
-                    float2 am = make_float2(0.0f, 0.0f);
-                    for (int w = 0; w < kSplitWarps; ++w) {
-                        const float2 v = ctl->amax[seq % kDoneSlots][w];
-                        am.x = fmaxf(am.x, v.x);
-                        am.y = fmaxf(am.y, v.y);
-                    }
-                    // Within these bounds the parts of everything down to 2^-30 of an operand's largest value are normal
-                    // numbers, and so are the products of the large values.
-                    constexpr float kTiny = 0x1p-80f, kHuge = 0x1p80f;
-                    const bool out_of_range = am.x > 0.0f && am.y > 0.0f &&
-                                              (am.x < kTiny || am.y < kTiny || am.x > kHuge || am.y > kHuge || am.x * am.y < kTiny);
                     float z = 0.0f;
 #pragma unroll
                     for (int j = 0; j < kCols; ++j) z = fmaf(acc[j], 0.0f, z);   // NaN if one of them is not finite
@@ -417,7 +447,7 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
                         else if (row < p.m) p.dbias[row] = (p.dbias_beta != 0.0f ? p.dbias_beta * p.dbias[row] : 0.0f) + sum;
                     }
                     const int64_t n0 = static_cast<int64_t>(at.n_tile) * BN + half * kCols;
-                    if (__any_sync(0xffffffffu, out_of_range || z != 0.0f)) {
+                    if (__any_sync(0xffffffffu, z != 0.0f)) {
                         int64_t row = static_cast<int64_t>(at.m_tile) * kBM + quarter * 32 + lane;
                         if (row >= p.m) row = p.m - 1;
                         const float* a = at.a + (AM ? row + kbeg * p.lda : row * p.lda + kbeg);
@@ -437,6 +467,9 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
                             a += a_step;
                             b += b_step;
                         }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kCols; ++j) acc[j] *= kDown;
                     }
                 }
                 tc_fence_before_thread_sync();

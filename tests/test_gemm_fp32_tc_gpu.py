@@ -132,3 +132,44 @@ def test_values_the_parts_cannot_carry(m, n, k):
     # an operand of zeros
     c, ref = check(a0 * 0.0, b)
     assert bool((c == 0).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 3072, 300), (256, 768, 3072)])
+@pytest.mark.parametrize("ta,tb", [(0, 1), (1, 0)])
+def test_rows_and_columns_of_any_size_side_by_side(m, n, k, ta, tb):
+    """Every row and every column keeps its own precision, down to subnormal values, whatever size its neighbours in the tile
+    have: the error of the block of each pair of sizes against its own norm.  Sums in the subnormal range are spaced 2^-149
+    apart: half of that for the product's result and for each of the k additions that an FMA chain would make there."""
+    a, b = _operands(m, n, k, ta, tb)
+    rows, cols = (0, -55, -110, -116, -124, -140), (0, -55, -100, 60, -124)
+    ra, cb = torch.arange(m, device=DEV) % len(rows), torch.arange(n, device=DEV) % len(cols)
+    sa, sb = torch.tensor([2.0 ** e for e in rows], device=DEV)[ra], torch.tensor([2.0 ** e for e in cols], device=DEV)[cb]
+    a, b = (a * sa if ta else a * sa[:, None]), (b * sb[:, None] if tb else b * sb)
+    c = torch.empty(m, n, device=DEV)
+    L.gemm(c, a, b, bool(ta), bool(tb))
+    ref = _product(a, b, ta, tb)
+    assert bool(torch.isfinite(c).all())
+    for i in range(len(rows)):
+        for j in range(len(cols)):
+            got, want = c[ra == i][:, cb == j].double(), ref[ra == i][:, cb == j]
+            spacing = 2.0 ** -150 * k * want.numel() ** 0.5
+            assert (got - want).norm().item() <= 8.0 * k ** 0.5 * 2.0 ** -24 * want.norm().item() + spacing, (rows[i], cols[j])
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 3072, 300), (256, 768, 3072)])
+def test_sums_near_the_largest_value(m, n, k):
+    """Products and sums beyond what the scaled parts can carry, none of them beyond fp32: rows of 2^60 times columns of
+    2^20 and 2^55, and a value of 2^110 among ordinary ones."""
+    a, b = _operands(m, n, k, 0, 1)
+    a[m // 2:] *= 2.0 ** 60
+    b *= 2.0 ** 20
+    b[n // 3:] *= 2.0 ** 35
+    a[7, 3] = 2.0 ** 110
+    b[:, 3] = 1.0
+    c = torch.empty(m, n, device=DEV)
+    L.gemm(c, a, b, False, True)
+    ref = _product(a, b, 0, 1)
+    assert bool(torch.isfinite(c).all())
+    for rows in (slice(0, 7), slice(7, 8), slice(8, m // 2), slice(m // 2, m)):
+        for cols in (slice(0, n // 3), slice(n // 3, n)):
+            assert _rel(c[rows, cols], ref[rows, cols]) <= 8.0 * k ** 0.5 * 2.0 ** -24
