@@ -952,7 +952,7 @@ bool plan_group(const llmt_b200_gemm_desc* descs, int count, TcPlan* plans) {
     return pairs;
 }
 
-int run_fp32(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b, cudaStream_t stream) {
+Fp32GemmParams fp32_params(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b) {
     Fp32GemmParams p{};
     p.m = d->m; p.n = d->n; p.k = d->k; p.batch = d->batch;
     p.a = static_cast<const float*>(a);
@@ -968,9 +968,14 @@ int run_fp32(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b
     p.alpha = d->alpha; p.beta = d->beta;
     p.bias = d->bias; p.bias_is_bf16 = d->bias_dtype == LLMT_B200_BF16;
     p.epi_flags = d->epilogue;
-    if (d->batch > 65535) return fail(LLMT_B200_ERR_UNSUPPORTED, "matmul: fp32 path supports batch <= 65535");
     p.dbias = d->dbias;
     p.dbias_beta = d->dbias_beta;
+    return p;
+}
+
+int run_fp32(const llmt_b200_gemm_desc* d, void* c, const void* a, const void* b, cudaStream_t stream) {
+    if (d->batch > 65535) return fail(LLMT_B200_ERR_UNSUPPORTED, "matmul: fp32 path supports batch <= 65535");
+    Fp32GemmParams p = fp32_params(d, c, a, b);
     p.wait_limit_ns = g_wait_limit_ns;
     p.status = device_status_ptr();
     if (p.status == nullptr) return fail(LLMT_B200_ERR_CUDA, "cannot resolve the device status word");
@@ -1534,8 +1539,13 @@ uint64_t llmt_b200_gemm_workspace_bytes_for(const llmt_b200_gemm_desc* d, const 
 int llmt_b200_gemm_plan(const llmt_b200_gemm_desc* d, char* buf, size_t n) {
     if (d == nullptr || buf == nullptr || n == 0) return fail(LLMT_B200_ERR_INVALID, "plan: null argument");
     if (d->dtype_ab != LLMT_B200_BF16) {
-        snprintf(buf, n, "fp32-simt tile=64x64x16 grid=%lldx%lldx%lld",
-                 (long long)((d->n + 63) / 64), (long long)((d->m + 63) / 64), (long long)d->batch);
+        const Fp32Plan pl = fp32_plan(fp32_params(d, nullptr, nullptr, nullptr));
+        if (pl.tensor_cores)
+            snprintf(buf, n, "fp32-tcgen05 tile=%dx%dx64 parts=3 splits=%d tiles=%dx%d grid=%lld", pl.bm, pl.bn, pl.splits, pl.tiles_m, pl.tiles_n,
+                     (long long)pl.ctas);
+        else
+            snprintf(buf, n, "fp32-simt tile=%dx%d warps=%d splits=%d tiles=%dx%d grid=%lld", pl.bm, pl.bn, pl.warps, pl.splits, pl.tiles_m,
+                     pl.tiles_n, (long long)pl.ctas);
         return LLMT_B200_OK;
     }
     const TcPlan pl = plan_single(d);

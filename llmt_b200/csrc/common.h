@@ -300,10 +300,17 @@ int tc_stages(bool pairs, int bn);             // and how many of them a CTA has
 int tc_dbias_rows_per_cta(void);
 int tc_dbias_finish_per_cta(void);
 cudaError_t launch_fp32_gemm(const Fp32GemmParams& p, cudaStream_t stream);
-// The tensor-core form (gemm_fp32_sm100.cu): its tiling of a problem and estimated cycles (bn 0: not for it); the launch.
-struct Fp32TcPlan { int bn, splits; int64_t cost; };
-Fp32TcPlan fp32_tc_plan(const Fp32GemmParams& p);
-cudaError_t launch_fp32_tc(const Fp32GemmParams& p, const Fp32TcPlan& plan, cudaStream_t stream);
+// How an fp32 problem runs: on the tensor cores (gemm_fp32_sm100.cu) or as one of the FMA forms (gemm_fp32_simt.cu), its tiles
+// and splits, the CTAs of the launch and the estimated cycles.
+struct Fp32Plan {
+    int tensor_cores, bm, bn, warps, splits;   // warps: of the FMA forms
+    int32_t tiles_m, tiles_n;
+    int64_t k_per_split, ctas, cost;
+};
+Fp32Plan fp32_plan(const Fp32GemmParams& p);
+// The tensor-core form: its plan (tensor_cores 0: not for it) and its launch.
+Fp32Plan fp32_tc_plan(const Fp32GemmParams& p);
+cudaError_t launch_fp32_tc(const Fp32GemmParams& p, const Fp32Plan& plan, cudaStream_t stream);
 cudaError_t launch_zero_f32(float* dst, int64_t n, cudaStream_t stream);
 cudaError_t launch_repack_bf16(RepackJobs jobs, cudaStream_t stream);
 cudaError_t launch_softmax_fwd(void* y, const void* x, int64_t rows, int64_t tq, int64_t tk,

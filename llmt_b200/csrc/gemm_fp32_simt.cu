@@ -751,17 +751,9 @@ int64_t fp32_cost(const F32Form& f, int64_t ctas, int64_t depth, int splits) {
 
 }  // namespace
 
-cudaError_t launch_fp32_gemm(const Fp32GemmParams& in, cudaStream_t stream) {
-    Fp32GemmParams p = in;
-    auto aligned = [&](const void* x, int64_t ld, int64_t stride, int64_t outer) {
-        return (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && ld % 4 == 0 && stride % 4 == 0 && (p.batch_inner <= 0 || outer % 4 == 0);
-    };
-    p.vec_a = p.trans_a && aligned(p.a, p.lda, p.stride_a, p.stride_a_outer);
-    p.vec_b = !p.trans_b && aligned(p.b, p.ldb, p.stride_b, p.stride_b_outer);
-    p.vec_c = aligned(p.c, p.ldc, p.stride_c, p.stride_c_outer);
-    // Form and splits from the cost model: a pure function of the problem's sizes.
-    int64_t best = 0;
-    int form = 0;
+Fp32Plan fp32_plan(const Fp32GemmParams& p) {
+    // Form and splits from the cost models: a pure function of the problem's sizes.
+    Fp32Plan best{};
     for (int i = 0; i < 3; ++i) {
         const F32Form& f = kF32Forms[i];
         const int64_t tm = (p.m + f.bm - 1) / f.bm, tn = (p.n + f.bn - 1) / f.bn;
@@ -770,23 +762,36 @@ cudaError_t launch_fp32_gemm(const Fp32GemmParams& in, cudaStream_t stream) {
             const int64_t sps = (steps + s - 1) / s;
             if (s > 1 && sps < 2) break;
             const int64_t cost = fp32_cost(f, tm * tn * p.batch * s, sps * kF32K, s);
-            if (best == 0 || cost < best) {
-                best = cost;
-                form = i;
-                p.splits = s;
-                p.k_per_split = sps * kF32K * f.groups;
-                p.tiles_m = static_cast<int32_t>(tm);
-                p.tiles_n = static_cast<int32_t>(tn);
+            if (best.cost == 0 || cost < best.cost) {
+                best = Fp32Plan{0, f.bm, f.bn, f.warps, s, static_cast<int32_t>(tm), static_cast<int32_t>(tn), sps * kF32K * f.groups,
+                                tm * tn * p.batch * s, cost};
             }
         }
     }
-    const Fp32TcPlan tc = fp32_tc_plan(in);
     // The tensor-core form where its model says so: both models count cycles and are pure functions of the sizes.  With few
     // rows or a short reduction a tile of 128 rows and its start cost more than the FMAs save (32 x 768 x 768: 8.6 us here,
     // 11.1 us there; 1000 x 100 x 100: 7.4 and 8.9), everything larger gains (256 x 256 x 64, 48 times: 17.7 and 15.2;
     // 256 x 2304 x 768: 36 and 16; 4096^3: 2780 and 830).
-    if (tc.bn != 0 && tc.cost < best) return launch_fp32_tc(in, tc, stream);
-    return form == 0 ? launch_fp32_size<2, 2, 1>(p, stream) : form == 1 ? launch_fp32_size<1, 2, 2>(p, stream) : launch_fp32_size<1, 2, 4>(p, stream);
+    const Fp32Plan tc = fp32_tc_plan(p);
+    return tc.tensor_cores && tc.cost < best.cost ? tc : best;
+}
+
+cudaError_t launch_fp32_gemm(const Fp32GemmParams& in, cudaStream_t stream) {
+    Fp32GemmParams p = in;
+    const Fp32Plan plan = fp32_plan(p);
+    p.tiles_m = plan.tiles_m;
+    p.tiles_n = plan.tiles_n;
+    p.splits = plan.splits;
+    p.k_per_split = plan.k_per_split;
+    if (plan.tensor_cores) return launch_fp32_tc(p, plan, stream);
+    auto aligned = [&](const void* x, int64_t ld, int64_t stride, int64_t outer) {
+        return (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && ld % 4 == 0 && stride % 4 == 0 && (p.batch_inner <= 0 || outer % 4 == 0);
+    };
+    p.vec_a = p.trans_a && aligned(p.a, p.lda, p.stride_a, p.stride_a_outer);
+    p.vec_b = !p.trans_b && aligned(p.b, p.ldb, p.stride_b, p.stride_b_outer);
+    p.vec_c = aligned(p.c, p.ldc, p.stride_c, p.stride_c_outer);
+    if (plan.bm == 128) return launch_fp32_size<2, 2, 1>(p, stream);
+    return plan.warps == 4 ? launch_fp32_size<1, 2, 2>(p, stream) : launch_fp32_size<1, 2, 4>(p, stream);
 }
 
 namespace {

@@ -643,13 +643,13 @@ constexpr int kTcSms = 148;
 
 }  // namespace
 
-Fp32TcPlan fp32_tc_plan(const Fp32GemmParams& p) {
-    Fp32TcPlan best{0, 1, 0};
+Fp32Plan fp32_tc_plan(const Fp32GemmParams& p) {
+    Fp32Plan best{};
     // A bias gradient of A stored [m, k] stays with the FMA kernel; the strict form of a tile must end within the waits.
     if (p.k < 1 || p.k > (1 << 20) || (p.dbias != nullptr && !p.trans_a)) return best;
-    const int64_t kblocks = (p.k + kBK - 1) / kBK;
+    const int64_t kblocks = (p.k + kBK - 1) / kBK, tiles_m = (p.m + kBM - 1) / kBM;
     for (int bn = 128; bn >= 64; bn -= 64) {
-        const int64_t tiles = ((p.m + kBM - 1) / kBM) * ((p.n + bn - 1) / bn) * p.batch;
+        const int64_t tiles_n = (p.n + bn - 1) / bn, tiles = tiles_m * tiles_n * p.batch;
         if (tiles > (1 << 28)) continue;
         for (int s = 1; s <= 8; s *= 2) {
             const int64_t per = (kblocks + s - 1) / s;
@@ -658,27 +658,24 @@ Fp32TcPlan fp32_tc_plan(const Fp32GemmParams& p) {
             const int64_t waves = (tiles * s + kTcSms - 1) / kTcSms;
             // cycles, fitted to 24 problems from 1 x 768 x 768 to 4096^3: a k-block, a tile's end, the launch and first loads
             const int64_t cost = waves * (per * (bn == 128 ? 3400 : 2500) + (bn == 128 ? 12000 : 4000)) + 9000 + (s > 1 ? 1500 : 0);
-            if (best.bn == 0 || cost < best.cost) best = Fp32TcPlan{bn, s, cost};
+            if (!best.tensor_cores || cost < best.cost) {
+                const int64_t ctas = s == 1 && tiles > kTcSms ? kTcSms : tiles * s;
+                best = Fp32Plan{1, kBM, bn, kTcThreads / 32, s, static_cast<int32_t>(tiles_m), static_cast<int32_t>(tiles_n), per * kBK, ctas, cost};
+            }
         }
     }
     return best;
 }
 
-cudaError_t launch_fp32_tc(const Fp32GemmParams& in, const Fp32TcPlan& plan, cudaStream_t stream) {
+cudaError_t launch_fp32_tc(const Fp32GemmParams& in, const Fp32Plan& plan, cudaStream_t stream) {
     Fp32GemmParams p = in;
-    const int64_t kblocks = (p.k + kBK - 1) / kBK;
-    p.tiles_m = static_cast<int32_t>((p.m + kBM - 1) / kBM);
-    p.tiles_n = static_cast<int32_t>((p.n + plan.bn - 1) / plan.bn);
-    p.splits = plan.splits;
-    p.k_per_split = (kblocks + plan.splits - 1) / plan.splits * kBK;
     auto aligned = [&](const void* x, int64_t ld, int64_t stride, int64_t outer) {
         return (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && ld % 4 == 0 && stride % 4 == 0 && (p.batch_inner <= 0 || outer % 4 == 0);
     };
     p.vec_a = aligned(p.a, p.lda, p.stride_a, p.stride_a_outer) && (!p.trans_a || p.m % 4 == 0);
     p.vec_b = aligned(p.b, p.ldb, p.stride_b, p.stride_b_outer) && (p.trans_b || p.n % 4 == 0);
     p.vec_c = aligned(p.c, p.ldc, p.stride_c, p.stride_c_outer);
-    const int64_t ctas = static_cast<int64_t>(p.tiles_m) * p.tiles_n * p.batch * p.splits;
-    const unsigned grid = static_cast<unsigned>(p.splits == 1 && ctas > kTcSms ? kTcSms : ctas);
+    const unsigned grid = static_cast<unsigned>(plan.ctas);
     return plan.bn == 128 ? launch_tc_size<128>(p, grid, stream) : launch_tc_size<64>(p, grid, stream);
 }
 

@@ -433,3 +433,14 @@ def test_a_grouped_bf16_result_keeps_its_parts(m, i, o):
         assert L.lib().llmt_b200_gemm_grouped_workspace_bytes((L.GemmDesc * 2)(dx, dw), 2, out) == L.OK
         return out[0]
     assert dx_bytes(L.BF16) == dx_bytes(L.FP32) > m * i * 4
+
+
+@pytest.mark.parametrize("m,n,k,kw,want", [
+    (256, 3072, 768, {}, "fp32-tcgen05 tile=128x128x64 parts=3 splits=2 tiles=2x24 grid=96"),
+    (4096, 4096, 4096, {}, "fp32-tcgen05 tile=128x128x64 parts=3 splits=1 tiles=32x32 grid=148"),      # walked persistently
+    (32, 768, 768, {}, "fp32-simt tile=64x64 warps=4 splits=8 tiles=1x12 grid=96"),
+    (4096, 4096, 512, dict(dbias=0x5000000), "fp32-simt tile=128x64 warps=4 splits=1 tiles=32x64 grid=2048"),   # op(A) summed along its rows
+])
+def test_the_plan_of_an_fp32_product_is_the_one_that_runs(m, n, k, kw, want):
+    d = _desc(m=m, n=n, k=k, lda=k, ldb=k, ldc=n, dtype_ab=L.FP32, dtype_c=L.FP32, **kw)
+    assert L.plan(d) == want and L.workspace_bytes(d) == 0
