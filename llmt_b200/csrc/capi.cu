@@ -85,10 +85,9 @@ int sm_count() {
         if (cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
             cached = n;
-        else
-            return 148;  // B200; used only for planning queries made without a device
     }
-    return g_sm_budget > 0 && g_sm_budget < cached ? g_sm_budget : cached;
+    const int all = cached > 0 ? cached : 148;   // B200, for planning queries made without a device
+    return g_sm_budget > 0 && g_sm_budget < all ? g_sm_budget : all;
 }
 
 // Cost of one 64-deep k-block of a tile in SM cycles.  Two bounds: the tensor pipe (2*bn
@@ -970,6 +969,7 @@ Fp32GemmParams fp32_params(const llmt_b200_gemm_desc* d, void* c, const void* a,
     p.epi_flags = d->epilogue;
     p.dbias = d->dbias;
     p.dbias_beta = d->dbias_beta;
+    p.sms = sm_count();
     return p;
 }
 

@@ -198,6 +198,7 @@ struct Fp32GemmParams {
     int32_t epi_flags;
     float* dbias;               // fp32 [m] or null: dbias[i] = dbias_beta * dbias[i] + sum_k op(A)[i, k]
     float dbias_beta;
+    int32_t sms;                // SMs that the launch is planned for and that a persistent grid stays within
     // Filled in by launch_fp32_gemm: the launch's tiling and which operands allow 16-byte accesses.
     int32_t tiles_m, tiles_n, splits;
     int64_t k_per_split;

@@ -743,8 +743,8 @@ constexpr F32Form kF32Forms[3] = {{128, 64, 4, 1, 94, 3600, 3700, 0},
 // problems (from 8 x 320 x 64 to 4096^3, four batched ones among them) in all forms and splits; its choice is
 // within 2 % of the best of them in the geometric mean and within 14 % at the worst.  Splits are powers of
 // two: clusters of 3 and 6 measured slower than either neighbour.
-int64_t fp32_cost(const F32Form& f, int64_t ctas, int64_t depth, int splits) {
-    const int64_t per_sm = (ctas + 147) / 148;
+int64_t fp32_cost(const F32Form& f, int64_t ctas, int64_t depth, int splits, int sms) {
+    const int64_t per_sm = (ctas + sms - 1) / sms;
     const int64_t per_k = per_sm * f.warps * f.step / 4;
     return depth * (per_k > 127 ? per_k : 127) + per_sm * f.tile + f.fixed + (splits > 1 ? 1300 + per_sm * splits * f.add : 0);
 }
@@ -752,7 +752,7 @@ int64_t fp32_cost(const F32Form& f, int64_t ctas, int64_t depth, int splits) {
 }  // namespace
 
 Fp32Plan fp32_plan(const Fp32GemmParams& p) {
-    // Form and splits from the cost models: a pure function of the problem's sizes.
+    // Form and splits from the cost models: a pure function of the problem's sizes and the SMs it may have.
     Fp32Plan best{};
     for (int i = 0; i < 3; ++i) {
         const F32Form& f = kF32Forms[i];
@@ -761,7 +761,7 @@ Fp32Plan fp32_plan(const Fp32GemmParams& p) {
         for (int s = 1; s <= 8; s *= 2) {
             const int64_t sps = (steps + s - 1) / s;
             if (s > 1 && sps < 2) break;
-            const int64_t cost = fp32_cost(f, tm * tn * p.batch * s, sps * kF32K, s);
+            const int64_t cost = fp32_cost(f, tm * tn * p.batch * s, sps * kF32K, s, p.sms);
             if (best.cost == 0 || cost < best.cost) {
                 best = Fp32Plan{0, f.bm, f.bn, f.warps, s, static_cast<int32_t>(tm), static_cast<int32_t>(tn), sps * kF32K * f.groups,
                                 tm * tn * p.batch * s, cost};

@@ -249,7 +249,7 @@ __device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst
     else pass(std::integral_constant<int, kLoadEdge>{});
 }
 
-// Grid: min(tiles, SMs) CTAs, or tiles * splits in clusters of `splits`.
+// Grid: min(tiles, the SMs that the caller leaves to it) CTAs, or tiles * splits in clusters of `splits`.
 template <int BN, bool AM, bool BMn>
 __global__ void __launch_bounds__(kTcThreads, 1)
 fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
@@ -639,8 +639,6 @@ cudaError_t launch_tc_size(const Fp32GemmParams& p, unsigned grid, cudaStream_t 
     return p.trans_b ? launch_tc_form<BN, true, false>(p, grid, stream) : launch_tc_form<BN, true, true>(p, grid, stream);
 }
 
-constexpr int kTcSms = 148;
-
 }  // namespace
 
 Fp32Plan fp32_tc_plan(const Fp32GemmParams& p) {
@@ -654,12 +652,13 @@ Fp32Plan fp32_tc_plan(const Fp32GemmParams& p) {
         for (int s = 1; s <= 8; s *= 2) {
             const int64_t per = (kblocks + s - 1) / s;
             // (how many clusters are resident at once: 144 CTAs in clusters of four, or 128 in clusters of eight, take two turns)
-            if (s > 1 && (tiles * s > (s == 2 ? 148 : s == 4 ? 128 : 112) || per < 2 || per * (s - 1) >= kblocks)) break;
-            const int64_t waves = (tiles * s + kTcSms - 1) / kTcSms;
+            const int most = s == 2 ? 148 : s == 4 ? 128 : 112;
+            if (s > 1 && (tiles * s > (most < p.sms ? most : p.sms) || per < 2 || per * (s - 1) >= kblocks)) break;
+            const int64_t waves = (tiles * s + p.sms - 1) / p.sms;
             // cycles, fitted to 24 problems from 1 x 768 x 768 to 4096^3: a k-block, a tile's end, the launch and first loads
             const int64_t cost = waves * (per * (bn == 128 ? 3400 : 2500) + (bn == 128 ? 12000 : 4000)) + 9000 + (s > 1 ? 1500 : 0);
             if (!best.tensor_cores || cost < best.cost) {
-                const int64_t ctas = s == 1 && tiles > kTcSms ? kTcSms : tiles * s;
+                const int64_t ctas = s == 1 && tiles > p.sms ? p.sms : tiles * s;
                 best = Fp32Plan{1, kBM, bn, kTcThreads / 32, s, static_cast<int32_t>(tiles_m), static_cast<int32_t>(tiles_n), per * kBK, ctas, cost};
             }
         }

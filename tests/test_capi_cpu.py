@@ -444,3 +444,17 @@ def test_a_grouped_bf16_result_keeps_its_parts(m, i, o):
 def test_the_plan_of_an_fp32_product_is_the_one_that_runs(m, n, k, kw, want):
     d = _desc(m=m, n=n, k=k, lda=k, ldb=k, ldc=n, dtype_ab=L.FP32, dtype_c=L.FP32, **kw)
     assert L.plan(d) == want and L.workspace_bytes(d) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(4096, 4096, 4096), (512, 50257, 768), (50257, 768, 512), (256, 3072, 768), (512, 768, 50257)])
+def test_fp32_products_on_the_tensor_cores_stay_within_the_sm_budget(m, n, k):
+    # persistent CTAs of 180 KB and more of shared memory, or one cluster of CTAs per tile: an SM has room for one of them
+    d = _desc(m=m, n=n, k=k, lda=k, ldb=k, ldc=n, dtype_ab=L.FP32, dtype_c=L.FP32)
+    whole = L.plan(d)
+    prev = L.set_sm_budget(100)
+    try:
+        plan = L.plan(d)
+        assert "fp32-tcgen05" in plan and int(re.search(r"grid=(\d+)", plan).group(1)) <= 100
+    finally:
+        L.set_sm_budget(prev)
+    assert L.plan(d) == whole

@@ -173,3 +173,17 @@ def test_sums_near_the_largest_value(m, n, k):
     for rows in (slice(0, 7), slice(7, 8), slice(8, m // 2), slice(m // 2, m)):
         for cols in (slice(0, n // 3), slice(n // 3, n)):
             assert _rel(c[rows, cols], ref[rows, cols]) <= 8.0 * k ** 0.5 * 2.0 ** -24
+
+
+def test_a_smaller_grid_gives_the_same_sums():
+    """Tiles walked by 40 CTAs instead of all: the splits are the same, hence the bits."""
+    a, b = _operands(1500, 1300, 700, 0, 1)
+    c, d = torch.empty(1500, 1300, device=DEV), torch.empty(1500, 1300, device=DEV)
+    L.gemm(c, a, b, False, True)
+    prev = L.set_sm_budget(40)
+    try:
+        assert "splits=1 " in L.plan(L.make_desc(d, a, b, False, True)) and "grid=40" in L.plan(L.make_desc(d, a, b, False, True))
+        L.gemm(d, a, b, False, True)
+    finally:
+        L.set_sm_budget(prev)
+    assert torch.equal(c, d)
