@@ -9,6 +9,7 @@
 // messages.  Both fill in the same descriptor and call the same C entry point.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -423,31 +424,87 @@ static const struct { const char* name; FastFn fn; } kFast[] = {
     ROW(gemm_softmax_bwd), ROW(rowdot), ROW(head_split), ROW(head_merge), ROW(cross_entropy_fwd), ROW(cross_entropy_bwd),
     ROW(lm_head_ce_fwd), ROW(lm_head_ce_bwd)};
 
+// What stands in the Python function's place: calls go to the native function, every attribute that it does not have itself
+// is the Python function's, and it is pickled by name as a function is.
+typedef struct {
+    PyObject_HEAD
+    vectorcallfunc vectorcall;
+    FastFn fn;
+    PyObject *slow, *dict, *weak;
+} Fast;
+static PyObject* fast_vectorcall(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kw) {
+    Fast* f = (Fast*)self;
+    return f->fn(f->slow, args, PyVectorcall_NARGS(nargsf), kw);
+}
+static PyObject* fast_getattro(PyObject* self, PyObject* name) {
+    PyObject* r = PyObject_GenericGetAttr(self, name);
+    if (r != NULL || !PyErr_ExceptionMatches(PyExc_AttributeError)) return r;
+    PyErr_Clear();
+    return PyObject_GetAttr(((Fast*)self)->slow, name);
+}
+static PyObject* fast_descr_get(PyObject* self, PyObject* obj, PyObject* type) {
+    (void)type;
+    if (obj == NULL || obj == Py_None) { Py_INCREF(self); return self; }
+    return PyMethod_New(self, obj);
+}
+static PyObject* fast_repr(PyObject* self) { return PyUnicode_FromFormat("<native form of %R>", ((Fast*)self)->slow); }
+static PyObject* fast_reduce(PyObject* self, PyObject* unused) {
+    (void)unused;
+    return PyObject_GetAttrString(self, "__qualname__");
+}
+static int fast_traverse(PyObject* self, visitproc visit, void* arg) {
+    Py_VISIT(((Fast*)self)->slow);
+    Py_VISIT(((Fast*)self)->dict);
+    return 0;
+}
+static int fast_clear(PyObject* self) {
+    Py_CLEAR(((Fast*)self)->dict);
+    return 0;
+}
+static void fast_dealloc(PyObject* self) {
+    PyObject_GC_UnTrack(self);
+    if (((Fast*)self)->weak != NULL) PyObject_ClearWeakRefs(self);
+    fast_clear(self);
+    Py_CLEAR(((Fast*)self)->slow);
+    PyObject_GC_Del(self);
+}
+static PyMethodDef kFastMethods[] = {{"__reduce__", fast_reduce, METH_NOARGS, NULL}, {NULL, NULL, 0, NULL}};
+static PyGetSetDef kFastGetSet[] = {{"__dict__", PyObject_GenericGetDict, PyObject_GenericSetDict, NULL, NULL}, {NULL, NULL, NULL, NULL, NULL}};
+static PyTypeObject FastType = {
+    PyVarObject_HEAD_INIT(NULL, 0)
+    .tp_name = "llmt_b200._native.Function", .tp_basicsize = sizeof(Fast),
+    .tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_HAVE_VECTORCALL,
+    .tp_vectorcall_offset = offsetof(Fast, vectorcall), .tp_call = PyVectorcall_Call, .tp_getattro = fast_getattro,
+    .tp_setattro = PyObject_GenericSetAttr, .tp_dictoffset = offsetof(Fast, dict), .tp_weaklistoffset = offsetof(Fast, weak),
+    .tp_descr_get = fast_descr_get, .tp_repr = fast_repr, .tp_methods = kFastMethods, .tp_getset = kFastGetSet,
+    .tp_traverse = fast_traverse, .tp_clear = fast_clear, .tp_dealloc = fast_dealloc};
+
 // fast(python_function): the native function of that name, with the Python one behind it.
 static PyObject* py_fast(PyObject* self, PyObject* slow) {
     (void)self;
     PyObject* name = PyObject_GetAttrString(slow, "__name__");
-    PyObject* doc = PyObject_GetAttrString(slow, "__doc__");
-    PyObject* r = NULL;
     const char* text = name != NULL ? PyUnicode_AsUTF8(name) : NULL;
+    Fast* r = NULL;
     for (size_t i = 0; text != NULL && r == NULL && i < sizeof(kFast) / sizeof(kFast[0]); ++i) {
         if (strcmp(text, kFast[i].name) != 0) continue;
-        PyMethodDef* def = (PyMethodDef*)PyMem_Calloc(1, sizeof *def);   // lives as long as the function: the process
-        if (def == NULL) { PyErr_NoMemory(); break; }
-        def->ml_name = kFast[i].name;
-        def->ml_meth = (PyCFunction)(void (*)(void))kFast[i].fn;
-        def->ml_flags = METH_FASTCALL | METH_KEYWORDS;
-        const char* d = doc != NULL && doc != Py_None ? PyUnicode_AsUTF8(doc) : NULL;
-        if (d != NULL) {
-            char* copy = (char*)PyMem_Malloc(strlen(d) + 1);
-            if (copy != NULL) def->ml_doc = strcpy(copy, d);
-        }
-        r = PyCFunction_NewEx(def, slow, NULL);
+        r = PyObject_GC_New(Fast, &FastType);
+        if (r == NULL) break;
+        r->vectorcall = fast_vectorcall;
+        r->fn = kFast[i].fn;
+        r->dict = r->weak = NULL;
+        Py_INCREF(slow);
+        r->slow = slow;
+        PyObject_GC_Track((PyObject*)r);
     }
     if (r == NULL && !PyErr_Occurred()) PyErr_Format(PyExc_ValueError, "no native function for %R", slow);
     Py_XDECREF(name);
-    Py_XDECREF(doc);
-    return r;
+    if (r == NULL) return NULL;
+    // its name, module, documentation, annotations and __wrapped__ (which gives it the signature)
+    PyObject* functools = PyImport_ImportModule("functools");
+    PyObject* wrapped = functools != NULL ? PyObject_CallMethod(functools, "update_wrapper", "OO", (PyObject*)r, slow) : NULL;
+    Py_XDECREF(functools);
+    Py_DECREF(r);
+    return wrapped;
 }
 
 // setup(binder, raise, scratch): what the native functions call back into.
@@ -485,6 +542,7 @@ static PyMethodDef kMethods[] = {{"fast", py_fast, METH_O, "The native form of a
 static struct PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Native call path of llmt_b200.", -1, kMethods, NULL, NULL, NULL, NULL};
 
 PyMODINIT_FUNC PyInit__native(void) {
+    if (PyType_Ready(&FastType) < 0) return NULL;
     PyObject* m = PyModule_Create(&kModule);
     if (m == NULL) return NULL;
     s_data_ptr = PyUnicode_InternFromString("data_ptr");
