@@ -519,7 +519,7 @@ def _bind_native() -> None:
     import torch
     entries = lib()
     _native.bind(tuple(ctypes.cast(getattr(entries, "llmt_b200_" + n), ctypes.c_void_p).value for n in _native.NAMES),
-                 torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.float32, torch.bfloat16, torch.int32)
+                 torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.float32, torch.bfloat16, torch.int32, GemmDesc)
 
 
 def _scratch(nbytes: int, like):

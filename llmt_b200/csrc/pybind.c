@@ -44,6 +44,7 @@ static int g_bound = 0;
 static PyObject *g_binder, *g_raise, *g_scratch;            // Python: loads the library; raises for a status; allocates scratch
 static PyObject *g_raw_stream, *g_get_device;               // torch's current stream handle of a device, and its current device
 static PyObject *g_float32, *g_bfloat16, *g_int32;
+static PyObject* g_desc_type;                               // the ctypes structure GemmDesc
 static PyObject *s_data_ptr, *s_shape, *s_stride, *s_dtype, *s_cuda_stream, *s_nbytes;
 
 static int ensure_bound(void) {
@@ -129,6 +130,7 @@ static int as_stream(PyObject* o, void** out) {
 }
 static int as_desc(PyObject* o, llmt_b200_gemm_desc* out) {   // a ctypes GemmDesc
     Py_buffer b;
+    if (!PyObject_TypeCheck(o, (PyTypeObject*)g_desc_type)) return -1;
     if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) < 0) { PyErr_Clear(); return -1; }
     const int ok = b.len == (Py_ssize_t)sizeof *out;
     if (ok) memcpy(out, b.buf, sizeof *out);
@@ -517,11 +519,11 @@ static PyObject* py_setup(PyObject* self, PyObject* args) {
     Py_RETURN_NONE;
 }
 
-// bind(addresses in the order of NAMES, torch's raw-stream and device getters, float32, bfloat16, int32)
+// bind(addresses in the order of NAMES, torch's raw-stream and device getters, float32, bfloat16, int32, GemmDesc)
 static PyObject* py_bind(PyObject* self, PyObject* args) {
     (void)self;
-    PyObject *list, *rs, *gd, *f, *h, *i32;
-    if (!PyArg_ParseTuple(args, "O!OOOOO", &PyTuple_Type, &list, &rs, &gd, &f, &h, &i32)) return NULL;
+    PyObject *list, *rs, *gd, *f, *h, *i32, *desc;
+    if (!PyArg_ParseTuple(args, "O!OOOOOO!", &PyTuple_Type, &list, &rs, &gd, &f, &h, &i32, &PyType_Type, &desc)) return NULL;
     if (PyTuple_GET_SIZE(list) != N_ENTRIES) return PyErr_Format(PyExc_ValueError, "bind: %zd addresses expected", N_ENTRIES);
     void* p[sizeof(kNames) / sizeof(kNames[0])];
     for (Py_ssize_t i = 0; i < N_ENTRIES; ++i) {
@@ -529,8 +531,8 @@ static PyObject* py_bind(PyObject* self, PyObject* args) {
         if (p[i] == NULL) return PyErr_Occurred() ? NULL : PyErr_Format(PyExc_ValueError, "bind: null address for %s", kNames[i]);
     }
     memcpy(&E, p, sizeof E);
-    Py_INCREF(rs); Py_INCREF(gd); Py_INCREF(f); Py_INCREF(h); Py_INCREF(i32);
-    g_raw_stream = rs; g_get_device = gd; g_float32 = f; g_bfloat16 = h; g_int32 = i32;
+    Py_INCREF(rs); Py_INCREF(gd); Py_INCREF(f); Py_INCREF(h); Py_INCREF(i32); Py_INCREF(desc);
+    g_raw_stream = rs; g_get_device = gd; g_float32 = f; g_bfloat16 = h; g_int32 = i32; g_desc_type = desc;
     g_bound = 1;
     Py_RETURN_NONE;
 }

@@ -26,3 +26,28 @@ def test_native_functions_keep_their_python_face(name):
         f.no_such_attribute
     holder = type("Holder", (), {"call": f})()
     assert holder.call.__self__ is holder and holder.call.__func__ is f
+
+
+class _At:
+    """Stands for a tensor, or a stream, of which only the address is asked."""
+    cuda_stream = 0
+
+    def __init__(self, at=0x1000):
+        self.at = at
+
+    def data_ptr(self):
+        return self.at
+
+
+def test_a_descriptor_is_a_descriptor():
+    """Bytes of the right length are not taken for one, a class derived from it is (m = 0: nothing is launched)."""
+    import ctypes
+    d = L.GemmDesc()
+    d.n = d.k = d.lda = d.ldb = d.ldc = d.batch = 1
+    raw = bytes(d)
+    for wrong in (raw, bytearray(raw), (ctypes.c_char * len(raw))(*raw)):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            L.gemm_desc(wrong, _At(0x1000), _At(0x2000), _At(0x3000), _At())
+    derived = type("Mine", (L.GemmDesc,), {}).from_buffer_copy(raw)
+    for right in (d, derived):
+        L.gemm_desc(right, _At(0x1000), _At(0x2000), _At(0x3000), _At())
