@@ -289,19 +289,30 @@ def gemm_desc(desc: GemmDesc, c, a, b, stream=None) -> None:
                                 _stream(stream)))
 
 
+def _group_array(index, element):
+    """An array of a Group whose address run() passes on: taken when the array is assigned, not on every run."""
+    def put(group, array):
+        ctypes.POINTER(element).from_param(array)   # what a call would take, or its TypeError
+        group._arrays[index] = array
+        group._at[index] = ctypes.cast(array, ctypes.c_void_p).value or 0
+    return property(lambda group: group._arrays[index], put)
+
+
 class Group:
     """A fixed list of independent bf16 problems launched as one kernel
     (llmt_b200_gemm_grouped). Built once from (desc, c, a, b) tuples; run() enqueues it."""
 
+    descs, c, a, b = _group_array(0, GemmDesc), _group_array(1, ctypes.c_void_p), _group_array(2, ctypes.c_void_p), _group_array(3, ctypes.c_void_p)
+
     def __init__(self, problems):
         n = len(problems)
         self.n = n
+        self._arrays, self._at = [None] * 4, [None] * 4
         self.descs = (GemmDesc * n)(*[p[0] for p in problems])
         self.tensors = [p[1:] for p in problems]  # keep the tensors alive
         self.c = (ctypes.c_void_p * n)(*[p[1].data_ptr() for p in problems])
         self.a = (ctypes.c_void_p * n)(*[p[2].data_ptr() for p in problems])
         self.b = (ctypes.c_void_p * n)(*[p[3].data_ptr() for p in problems])
-        self._at = tuple(ctypes.addressof(x) for x in (self.descs, self.c, self.a, self.b))
 
     def workspace_bytes(self):
         out = (ctypes.c_uint64 * self.n)()

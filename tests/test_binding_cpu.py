@@ -51,3 +51,20 @@ def test_a_descriptor_is_a_descriptor():
     derived = type("Mine", (L.GemmDesc,), {}).from_buffer_copy(raw)
     for right in (d, derived):
         L.gemm_desc(right, _At(0x1000), _At(0x2000), _At(0x3000), _At())
+
+
+def test_a_group_runs_the_arrays_it_has(monkeypatch):
+    import ctypes
+    seen = []
+    monkeypatch.setattr(L, "_group_run", lambda *args: seen.append(args))
+    g = L.Group([(L.GemmDesc(), _At(0x1000), _At(0x2000), _At(0x3000)), (L.GemmDesc(), _At(0x4000), _At(0x5000), _At(0x6000))])
+    g.run()
+    assert seen[0] == (*(ctypes.addressof(x) for x in (g.descs, g.c, g.a, g.b)), 2, None)
+    g.c = (ctypes.c_void_p * 2)(0x7000, 0x8000)
+    g.descs = (L.GemmDesc * 2)(*g.descs)
+    g.a = ctypes.cast(g.b, ctypes.POINTER(ctypes.c_void_p))
+    g.run()
+    assert seen[1] == (ctypes.addressof(g.descs), ctypes.addressof(g.c), ctypes.addressof(g.b), ctypes.addressof(g.b), 2, None)
+    assert list(g.c) == [0x7000, 0x8000]
+    with pytest.raises(TypeError):
+        g.b = [0x9000, 0xa000]
