@@ -9,6 +9,7 @@ the library is missing or a call fails, an exception is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -538,7 +539,7 @@ def _scratch(nbytes: int, like):
     return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
 
 
-if os.path.exists(os.path.join(_HERE, "_native.so")):
+if os.path.exists(os.path.join(_HERE, "_native" + importlib.machinery.EXTENSION_SUFFIXES[0])):   # built for this interpreter
     from . import _native
     _native.setup(_bind_native, _check, _scratch)
     for _f in (_group_run, gemm, gemm_desc, zero_grads, softmax_fwd, softmax_bwd, gemm_softmax_fwd, gemm_softmax_bwd, rowdot,

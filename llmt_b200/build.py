@@ -8,6 +8,7 @@ library to llmt_b200/lib/libllmt_b200.so.
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.machinery
 import os
 import shutil
 import subprocess
@@ -84,7 +85,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 NATIVE_SRC = os.path.join(CSRC, "pybind.c")
-NATIVE_PATH = os.path.join(HERE, "_native.so")
+NATIVE_PATH = os.path.join(HERE, "_native" + importlib.machinery.EXTENSION_SUFFIXES[0])   # for this interpreter only
 
 
 def build_native(force: bool = False) -> str:
@@ -93,12 +94,15 @@ def build_native(force: bool = False) -> str:
     if force or _stale(NATIVE_PATH, [NATIVE_SRC, header, os.path.abspath(__file__)]):
         cc = shutil.which("cc") or shutil.which("gcc")
         if cc is None:
-            raise RuntimeError("a C compiler is required to build llmt_b200/_native.so")
+            raise RuntimeError("a C compiler is required to build llmt_b200._native")
         cmd = [cc, "-std=c11", "-O2", "-Wall", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], NATIVE_SRC, "-o", NATIVE_PATH]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("the Python extension failed to build")
+    untagged = os.path.join(HERE, "_native.so")   # any interpreter would load that one
+    if os.path.exists(untagged):
+        os.remove(untagged)
     return NATIVE_PATH
 
 

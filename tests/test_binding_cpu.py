@@ -68,3 +68,12 @@ def test_a_group_runs_the_arrays_it_has(monkeypatch):
     assert list(g.c) == [0x7000, 0x8000]
     with pytest.raises(TypeError):
         g.b = [0x9000, 0xa000]
+
+
+def test_the_extension_belongs_to_one_interpreter():
+    import importlib.machinery
+    import os
+    from llmt_b200 import _native, build
+    tag = importlib.machinery.EXTENSION_SUFFIXES[0]
+    assert tag != ".so" and _native.__file__.endswith("_native" + tag) and os.path.samefile(_native.__file__, build.NATIVE_PATH)
+    assert not os.path.exists(os.path.join(os.path.dirname(_native.__file__), "_native.so"))
