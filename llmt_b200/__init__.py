@@ -358,6 +358,18 @@ def gemm_static_scratch(desc: GemmDesc, c, a, b, stream=None) -> None:
                                                b.data_ptr(), _stream(stream)))
 
 
+def _scratch(nbytes: int, like, stream=None):
+    """Scratch for one call on `stream` that may be let go once the call is enqueued: it comes from that stream's own
+    memory, so whoever gets it next is ordered after the call."""
+    import torch
+    if stream is None:
+        return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=like.device)
+    with torch.cuda.stream(stream):
+        return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
+
+
 def gemm(c, a, b, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, bias=None, gelu=False,
          dbias=None, dbias_beta=0.0, workspace=None, stream=None, tile_n=0, splits=0, cta_pairs=0) -> None:
     """C = epilogue(alpha*op(A)*op(B) + beta*C) on device tensors, in place in C.
@@ -366,13 +378,12 @@ def gemm(c, a, b, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, bias=None, 
     (include/llmt/kernels/matmul.h:12-24) plus the fused bias / GELU / dbias
     extensions. If the problem needs split-K scratch and none is passed, a
     torch buffer is allocated for this call."""
-    import torch
     d = make_desc(c, a, b, trans_a, trans_b, alpha, beta, bias, gelu, dbias, dbias_beta, workspace,
                   tile_n, splits, cta_pairs)
     if workspace is None:
         need = workspace_bytes(d, a, b)
         if need:
-            ws = torch.empty(need, dtype=torch.uint8, device=c.device)
+            ws = _scratch(need, c, stream)
             d.workspace = ws.data_ptr()
             d.workspace_bytes = need
     gemm_desc(d, c, a, b, stream)
@@ -532,11 +543,6 @@ def _bind_native() -> None:
     entries = lib()
     _native.bind(tuple(ctypes.cast(getattr(entries, "llmt_b200_" + n), ctypes.c_void_p).value for n in _native.NAMES),
                  torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.float32, torch.bfloat16, torch.int32, GemmDesc)
-
-
-def _scratch(nbytes: int, like):
-    import torch
-    return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
 
 
 if os.path.exists(os.path.join(_HERE, "_native" + importlib.machinery.EXTENSION_SUFFIXES[0])):   # built for this interpreter

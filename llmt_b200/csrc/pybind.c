@@ -268,7 +268,7 @@ FAST(gemm) {
         const uint64_t need = E.gemm_workspace_bytes_for(&d, a.ptr, b.ptr);
         if (need > 0) {
             PyObject* n = PyLong_FromUnsignedLongLong(need);
-            scratch = n != NULL ? PyObject_CallFunctionObjArgs(g_scratch, n, v[0], NULL) : NULL;
+            scratch = n != NULL ? PyObject_CallFunctionObjArgs(g_scratch, n, v[0], v[12] != NULL ? v[12] : Py_None, NULL) : NULL;
             Py_XDECREF(n);
             if (scratch == NULL) return NULL;   // out of memory: torch's own error
             if (as_ptr(scratch, &d.workspace) < 0) { Py_DECREF(scratch); SLOW(); }
