@@ -22,9 +22,9 @@
 // sixteen splitting warps with half the registers measured the same.  BN = 64 takes 2500 cycles for half the outputs and
 // serves problems with few tiles.
 //
-// Measured against the FMA kernel (us, and error against 64 bits): y = x W^T 256 x 3072 x 768 36.8 -> 21.5 (2.5e-7 ->
-// 1.0e-7), 512 x 50257 x 768 856 -> 310 (5.0e-7 -> 1.0e-7), dX of that layer 962 -> 400 (1.4e-6 -> 2.7e-7), its dW
-// 824 -> 383 (4.0e-7 -> 9.6e-8), 4096^3 2780 -> 830 (166 TFLOP/s).
+// Measured against the FMA kernel (us, and error against 64 bits): y = x W^T 256 x 3072 x 768 36.8 -> 20.7 (2.5e-7 ->
+// 1.0e-7), 512 x 50257 x 768 856 -> 294 (5.0e-7 -> 1.0e-7), dX of that layer 962 -> 402 (1.4e-6 -> 2.7e-7), its dW
+// 824 -> 359 (4.0e-7 -> 9.6e-8), 4096^3 2780 -> 832 (165 TFLOP/s).
 //
 // Range: both operands are multiplied by 2^24 before they are split and the sums by 2^-48 afterwards, both exact.  The last
 // bit of any fp32 value, subnormal ones too, is then at 2^-125 or above, so every part is a normal number, and what
@@ -150,13 +150,14 @@ __device__ __forceinline__ void load_operand(float4 (&v)[W / 16], LoadForm form,
     for (int u = 0; u < W / 16; ++u) v[u] = load_group<MN, W>(u, form, x, ld, r0, rows, k0, kend);
 }
 
+// Two values rounded to bf16, and each of them as a float again.
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 __device__ __forceinline__ float low_of(uint32_t h) { return __uint_as_float(h << 16); }
 __device__ __forceinline__ float high_of(uint32_t h) { return __uint_as_float(h & 0xFFFF0000u); }
-// The same on pairs of floats.
+// Arithmetic on pairs of floats.
 __device__ __forceinline__ uint64_t pair2(float lo, float hi) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -203,25 +204,11 @@ __device__ __forceinline__ void split_group(int u, const float4& x, uint32_t dst
     const uint32_t blk = MN ? ((tid % kLanes) >> 4) * (64u * 128u) : 0u;
     // (row & 7 is the same for all of a thread's groups)
     const uint32_t at = dst + blk + row * 128u + (((c >> 1) ^ (row & 7u)) << 4) + (c & 1u) * 8u + static_cast<uint32_t>(u) * (kStep * 128u);
-    uint32_t h0, h1, m0, m1, l0, l1;
-    if (PACKED) {
-        const uint64_t up = pair2(kUp, kUp), x0 = pair2(x.x, x.y), x1 = pair2(x.z, x.w);
-        h0 = round2(mul2(x0, up));
-        h1 = round2(mul2(x1, up));
-        const uint64_t r0 = fma2(x0, up, negated2(h0)), r1 = fma2(x1, up, negated2(h1));
-        m0 = round2(r0);
-        m1 = round2(r1);
-        l0 = round2(add2(r0, negated2(m0)));
-        l1 = round2(add2(r1, negated2(m1)));
-    } else {
-        h0 = pack2(x.x * kUp, x.y * kUp);
-        h1 = pack2(x.z * kUp, x.w * kUp);
-        const float r0 = fmaf(x.x, kUp, -low_of(h0)), r1 = fmaf(x.y, kUp, -high_of(h0)), r2 = fmaf(x.z, kUp, -low_of(h1)), r3 = fmaf(x.w, kUp, -high_of(h1));
-        m0 = pack2(r0, r1);
-        m1 = pack2(r2, r3);
-        l0 = pack2(r0 - low_of(m0), r1 - high_of(m0));
-        l1 = pack2(r2 - low_of(m1), r3 - high_of(m1));
-    }
+    const uint64_t up = pair2(kUp, kUp), x0 = pair2(x.x, x.y), x1 = pair2(x.z, x.w);
+    const uint32_t h0 = round2(mul2(x0, up)), h1 = round2(mul2(x1, up));
+    const uint64_t r0 = fma2(x0, up, negated2(h0)), r1 = fma2(x1, up, negated2(h1));
+    const uint32_t m0 = round2(r0), m1 = round2(r1);
+    const uint32_t l0 = round2(add2(r0, negated2(m0))), l1 = round2(add2(r1, negated2(m1)));
     st_shared8(at, h0, h1);
     st_shared8(at + kPart, m0, m1);
     st_shared8(at + 2 * kPart, l0, l1);
@@ -247,6 +234,71 @@ __device__ __forceinline__ void split_and_load(float4 (&v)[W / 16], uint32_t dst
     else if (form == kLoadVec) pass(std::integral_constant<int, kLoadVec>{});
     else if (form == kLoadScalar) pass(std::integral_constant<int, kLoadScalar>{});
     else pass(std::integral_constant<int, kLoadEdge>{});
+}
+
+// The sums of a warp's 32 x COLS outputs (lane = row) again, by fp32 FMAs in ascending k, from the operands as they are.
+// Four k at a time go through the warp's staging buffer while the next four are on their way.  Measured with one NaN in A,
+// us, and with single values loaded from global memory for every FMA instead: 256 x 3072 x 768 213 and 523, 512 x 50257 x
+// 768 4736 and 11847; the FMA kernel, whose time does not depend on the values, takes 37 and 856.
+struct Operand {
+    const float* x;
+    int64_t ld, first, rows;   // the m or n index: the block's first row, and how many there are (the last one repeats)
+};
+template <bool MN, int W>
+__device__ __forceinline__ void strict_fetch(float (&v)[W / 8], const Operand& o, int64_t k0, int64_t kend) {
+    const int lane = static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+    for (int i = 0; i < W / 8; ++i) {
+        const int e = lane + 32 * i;
+        const int64_t k = k0 + (MN ? e / W : e & 3);
+        int64_t row = o.first + (MN ? e % W : e >> 2);
+        if (row >= o.rows) row = o.rows - 1;
+        v[i] = k < kend ? o.x[MN ? k * o.ld + row : row * o.ld + k] : 0.0f;
+    }
+}
+template <bool MN, int W>
+__device__ __forceinline__ void strict_stage(const float (&v)[W / 8], float* to) {
+    const int lane = static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+    for (int i = 0; i < W / 8; ++i) {
+        const int e = lane + 32 * i;
+        to[(MN ? e / W : e & 3) * (W + 8) + (MN ? e % W : e >> 2)] = v[i];
+    }
+}
+template <bool AM, bool BMn, int COLS>
+__device__ __forceinline__ void strict_sums(float (&acc)[COLS], float* buf, const Operand& a, const Operand& b, int64_t kbeg, int64_t kend) {
+    constexpr int kPitchA = 32 + 8, kPitchB = COLS + 8;
+    static_assert(4 * (kPitchA + kPitchB) <= 32 * 16, "the warp's staging buffer");
+    float* const b_sm = buf + 4 * kPitchA;
+    const int lane = static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
+    float va[4], vb[COLS / 8];
+    strict_fetch<AM, 32>(va, a, kbeg, kend);
+    strict_fetch<BMn, COLS>(vb, b, kbeg, kend);
+#pragma unroll 1
+    for (int64_t k0 = kbeg; k0 < kend; k0 += 4) {
+        __syncwarp();   // (the buffer's readers are done)
+        strict_stage<AM, 32>(va, buf);
+        strict_stage<BMn, COLS>(vb, b_sm);
+        __syncwarp();
+        strict_fetch<AM, 32>(va, a, k0 + 4, kend);
+        strict_fetch<BMn, COLS>(vb, b, k0 + 4, kend);
+        const int steps = kend - k0 < 4 ? static_cast<int>(kend - k0) : 4;
+#pragma unroll 1
+        for (int k = 0; k < steps; ++k) {
+            const float av = buf[k * kPitchA + lane];
+#pragma unroll
+            for (int j = 0; j < COLS; j += 4) {
+                const float4 bv = *reinterpret_cast<const float4*>(b_sm + k * kPitchB + j);
+                acc[j] = fmaf(av, bv.x, acc[j]);
+                acc[j + 1] = fmaf(av, bv.y, acc[j + 1]);
+                acc[j + 2] = fmaf(av, bv.z, acc[j + 2]);
+                acc[j + 3] = fmaf(av, bv.w, acc[j + 3]);
+            }
+        }
+    }
+    __syncwarp();
 }
 
 // Grid: min(tiles, the SMs that the caller leaves to it) CTAs, or tiles * splits in clusters of `splits`.
@@ -448,25 +500,8 @@ fp32_tc_kernel(const __grid_constant__ Fp32GemmParams p) {
                     }
                     const int64_t n0 = static_cast<int64_t>(at.n_tile) * BN + half * kCols;
                     if (__any_sync(0xffffffffu, z != 0.0f)) {
-                        int64_t row = static_cast<int64_t>(at.m_tile) * kBM + quarter * 32 + lane;
-                        if (row >= p.m) row = p.m - 1;
-                        const float* a = at.a + (AM ? row + kbeg * p.lda : row * p.lda + kbeg);
-                        const int64_t a_step = AM ? p.lda : 1, b_step = BMn ? p.ldb : 1, b_col = BMn ? 1 : p.ldb;
-                        const float* b = at.b + kbeg * b_step + (n0 < p.n ? n0 : p.n - 1) * b_col;
-#pragma unroll
-                        for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
-#pragma unroll 1
-                        for (int64_t k = kbeg; k < kend; ++k) {
-                            const float av = *a;
-                            const float* bj = b;
-#pragma unroll
-                            for (int j = 0; j < kCols; ++j) {
-                                acc[j] = fmaf(av, *bj, acc[j]);
-                                if (n0 + j + 1 < p.n) bj += b_col;   // (columns beyond the matrix repeat its last one)
-                            }
-                            a += a_step;
-                            b += b_step;
-                        }
+                        const Operand oa{at.a, p.lda, static_cast<int64_t>(at.m_tile) * kBM + quarter * 32, p.m}, ob{at.b, p.ldb, n0, p.n};
+                        strict_sums<AM, BMn, kCols>(acc, buf, oa, ob, kbeg, kend);
                     } else {
 #pragma unroll
                         for (int j = 0; j < kCols; ++j) acc[j] *= kDown;

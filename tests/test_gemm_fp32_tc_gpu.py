@@ -187,3 +187,23 @@ def test_a_smaller_grid_gives_the_same_sums():
     finally:
         L.set_sm_budget(prev)
     assert torch.equal(c, d)
+
+
+# rows and columns at the ends of the matrix and of a warp's block, k that is no multiple of the four taken at a time
+@pytest.mark.parametrize("m,n,k", [(129, 3001, 130), (300, 500, 777), (256, 768, 3071)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_sums_formed_again_by_fmas(m, n, k, ta, tb):
+    """An infinity in the first and the last row and in a column sends every block that they cross through the FMA form; what
+    they do not touch there comes out as precise as an FMA chain makes it."""
+    a, b = _operands(m, n, k, ta, tb)
+    at, bt = (a.T if ta else a), (b.T if tb else b)
+    at[0, k - 1], at[m - 1, 0], bt[k // 2, n - 1] = float("inf"), -float("inf"), float("inf")
+    c = torch.empty(m, n, device=DEV)
+    L.gemm(c, a, b, bool(ta), bool(tb))
+    ref = _product(a, b, ta, tb)
+    assert torch.equal(torch.isinf(c), torch.isinf(ref)) and torch.equal(torch.isnan(c), torch.isnan(ref))
+    assert torch.equal(c[torch.isinf(c)].double(), ref[torch.isinf(ref)])
+    fine = torch.isfinite(ref)
+    assert int(fine.sum()) == (m - 2) * (n - 1)
+    assert _rel(c[fine], ref[fine]) <= 8.0 * k ** 0.5 * 2.0 ** -24
+    assert _rel(c[1:m - 1, :n - 1][:, -64:], ref[1:m - 1, :n - 1][:, -64:]) <= 8.0 * k ** 0.5 * 2.0 ** -24
