@@ -678,7 +678,8 @@ cudaError_t launch_tc_size(const Fp32GemmParams& p, unsigned grid, cudaStream_t 
 
 Fp32Plan fp32_tc_plan(const Fp32GemmParams& p) {
     Fp32Plan best{};
-    // A bias gradient of A stored [m, k] stays with the FMA kernel; the strict form of a tile must end within the waits.
+    // A bias gradient of A stored [m, k] stays with the FMA kernel; so do reductions whose FMA form (see launch_fp32_tc) would keep
+    // a CTA for more than a second.
     if (p.k < 1 || p.k > (1 << 20) || (p.dbias != nullptr && !p.trans_a)) return best;
     const int64_t kblocks = (p.k + kBK - 1) / kBK, tiles_m = (p.m + kBM - 1) / kBM;
     for (int bn = 128; bn >= 64; bn -= 64) {
@@ -709,6 +710,9 @@ cudaError_t launch_fp32_tc(const Fp32GemmParams& in, const Fp32Plan& plan, cudaS
     p.vec_a = aligned(p.a, p.lda, p.stride_a, p.stride_a_outer) && (!p.trans_a || p.m % 4 == 0);
     p.vec_b = aligned(p.b, p.ldb, p.stride_b, p.stride_b_outer) && (p.trans_b || p.n % 4 == 0);
     p.vec_c = aligned(p.c, p.ldc, p.stride_c, p.stride_c_outer);
+    // While a tile's sums are formed again by FMAs (at most 0.6 us per k, measured) the CTA's other warps wait for it: that time comes
+    // on top of what a caller allows a wait to take.
+    p.wait_limit_ns += static_cast<uint64_t>(p.k_per_split) * 2000u;
     const unsigned grid = static_cast<unsigned>(plan.ctas);
     return plan.bn == 128 ? launch_tc_size<128>(p, grid, stream) : launch_tc_size<64>(p, grid, stream);
 }

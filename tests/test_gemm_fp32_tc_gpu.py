@@ -207,3 +207,23 @@ def test_sums_formed_again_by_fmas(m, n, k, ta, tb):
     assert int(fine.sum()) == (m - 2) * (n - 1)
     assert _rel(c[fine], ref[fine]) <= 8.0 * k ** 0.5 * 2.0 ** -24
     assert _rel(c[1:m - 1, :n - 1][:, -64:], ref[1:m - 1, :n - 1][:, -64:]) <= 8.0 * k ** 0.5 * 2.0 ** -24
+
+
+def test_a_short_wait_limit_allows_for_sums_formed_again():
+    """25000 k per split take milliseconds when they are formed again by FMAs, with the other warps waiting: no reason to give up,
+    also where a caller allows a wait half a millisecond."""
+    k = 200000
+    a, b = _operands(128, 128, k, 0, 1)
+    a[5, 7] = float("nan")
+    c = torch.empty(128, 128, device=DEV)
+    L.gemm(c, a, b, False, True)
+    torch.cuda.synchronize()
+    L.set_wait_limit_ns(gemm_ns=500000)
+    try:
+        L.gemm(c, a, b, False, True)
+        assert L.device_status() == (0, 0)
+    finally:
+        L.set_wait_limit_ns(gemm_ns=2000000000)
+    ref = _product(a, b, 0, 1)
+    rows = torch.arange(128, device=DEV) != 5
+    assert bool(torch.isnan(c[5]).all()) and _rel(c[rows], ref[rows]) <= 8.0 * k ** 0.5 * 2.0 ** -24
