@@ -591,19 +591,28 @@ repack_bf16_kernel(const __grid_constant__ RepackJobs jobs) {
 
 // Head split / merge as copies (llmt include/llmt/kernels/permute.h:21-46).  The GEMMs can read
 // and write the per-head layout through strides, so these are only needed where a caller wants
-// the re-shelved tensor itself.  A block takes one token row at a time (no 64-bit division per element: that
-// bound the kernel at 9 us for 9.4 MB), a thread moves `vec` consecutive elements of one head's row
+// the re-shelved tensor itself.  `1 << shift` threads take a token row, as many as it has vectors up to the whole block
+// (131072 rows of 8 vectors merged: 5.4 us; with a whole block for every row 57 us), without a 64-bit division per
+// element (that bound the kernel at 9 us for 9.4 MB).  A thread moves `vec` consecutive elements of one head's row
 // (hd is a multiple of vec): 16 bytes when the pointers and hd allow it, else one element.
 //   merge: y[b, t, h*hd + d] = x[b, h, t, d]
 //   split: out[part][b, h, t, d] = qkv[b, t, part*A + h*hd + d],  A = H*hd, part = 0..parts-1
+__device__ __forceinline__ int64_t first_token(int shift) {
+    return static_cast<int64_t>(blockIdx.x) * (256 >> shift) + (threadIdx.x >> shift);
+}
+__device__ __forceinline__ int64_t token_step(int shift) { return static_cast<int64_t>(gridDim.x) * (256 >> shift); }
+__device__ __forceinline__ int64_t item_of(int64_t token, int64_t tokens, int64_t T) {
+    return tokens <= 0x7fffffff ? static_cast<int64_t>(static_cast<uint32_t>(token) / static_cast<uint32_t>(T)) : token / T;
+}
+
 template <typename V>
 __global__ void __launch_bounds__(256)
-head_merge_kernel(V* __restrict__ y, const V* x, int64_t tokens, uint32_t H, int64_t T, uint32_t hdv) {
+head_merge_kernel(V* __restrict__ y, const V* x, int64_t tokens, uint32_t H, int64_t T, uint32_t hdv, int shift) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t width = H * hdv;
-    for (int64_t token = blockIdx.x; token < tokens; token += gridDim.x) {
-        const int64_t b = token / T, t = token - b * T;
-        for (uint32_t i = threadIdx.x; i < width; i += 256u) {
+    for (int64_t token = first_token(shift); token < tokens; token += token_step(shift)) {
+        const int64_t b = item_of(token, tokens, T), t = token - b * T;
+        for (uint32_t i = threadIdx.x & ((1u << shift) - 1u); i < width; i += 1u << shift) {
             const uint32_t h = i / hdv, d = i - h * hdv;
             y[token * width + i] = x[((b * H + h) * T + t) * hdv + d];
         }
@@ -613,12 +622,12 @@ head_merge_kernel(V* __restrict__ y, const V* x, int64_t tokens, uint32_t H, int
 template <typename V>
 __global__ void __launch_bounds__(256)
 head_split_kernel(V* __restrict__ q, V* __restrict__ k, V* __restrict__ v, const V* qkv, int64_t tokens, uint32_t H, int64_t T,
-                  uint32_t hdv) {
+                  uint32_t hdv, int shift) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t width = H * hdv;
-    for (int64_t token = blockIdx.x; token < tokens; token += gridDim.x) {
-        const int64_t b = token / T, t = token - b * T;
-        for (uint32_t i = threadIdx.x; i < 3u * width; i += 256u) {
+    for (int64_t token = first_token(shift); token < tokens; token += token_step(shift)) {
+        const int64_t b = item_of(token, tokens, T), t = token - b * T;
+        for (uint32_t i = threadIdx.x & ((1u << shift) - 1u); i < 3u * width; i += 1u << shift) {
             const uint32_t head = i / hdv, d = i - head * hdv;   // over the heads of q, k and v
             const uint32_t part = head / H, h = head - part * H;
             V* out = part == 0 ? q : part == 1 ? k : v;
@@ -801,17 +810,28 @@ bool vec16_ok(std::initializer_list<const void*> ptrs, int64_t hd, int elem_byte
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;
     return true;
 }
-unsigned token_blocks(int64_t tokens) { return static_cast<unsigned>(tokens < 148 * 64 ? tokens : 148 * 64); }
+// Threads that share a token row of `vectors` (their number's logarithm), and the blocks for all rows.
+int token_shift(int64_t vectors) {
+    int shift = 0;
+    while (shift < 8 && (int64_t{1} << shift) < vectors) ++shift;
+    return shift;
+}
+unsigned token_blocks(int64_t tokens, int shift) {
+    const int64_t blocks = (tokens + (256 >> shift) - 1) / (256 >> shift);
+    return static_cast<unsigned>(blocks < 148 * 64 ? blocks : 148 * 64);
+}
 
 template <typename V>
 cudaError_t head_merge_as(void* y, const void* x, int64_t B, int64_t H, int64_t T, int64_t hdv, cudaStream_t stream) {
-    return launch_dependent(head_merge_kernel<V>, token_blocks(B * T), 256, stream, static_cast<V*>(y), static_cast<const V*>(x), B * T,
-                            static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv));
+    const int shift = token_shift(H * hdv);
+    return launch_dependent(head_merge_kernel<V>, token_blocks(B * T, shift), 256, stream, static_cast<V*>(y), static_cast<const V*>(x), B * T,
+                            static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv), shift);
 }
 template <typename V>
 cudaError_t head_split_as(void* q, void* k, void* v, const void* qkv, int64_t B, int64_t H, int64_t T, int64_t hdv, cudaStream_t stream) {
-    return launch_dependent(head_split_kernel<V>, token_blocks(B * T), 256, stream, static_cast<V*>(q), static_cast<V*>(k),
-                            static_cast<V*>(v), static_cast<const V*>(qkv), B * T, static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv));
+    const int shift = token_shift(3 * H * hdv);
+    return launch_dependent(head_split_kernel<V>, token_blocks(B * T, shift), 256, stream, static_cast<V*>(q), static_cast<V*>(k),
+                            static_cast<V*>(v), static_cast<const V*>(qkv), B * T, static_cast<uint32_t>(H), T, static_cast<uint32_t>(hdv), shift);
 }
 }  // namespace
 

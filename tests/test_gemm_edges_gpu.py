@@ -309,3 +309,17 @@ def test_repacked_copy_of_long_rows_stays_within_them(cols):
             assert torch.equal(x, y[:, :cols]) and bool((y[:, cols:] == 0).all())
         assert bool((ws[need:] == 0x5A).all())
     assert oracle.rel_fro(c.cpu().numpy(), oracle.gemm(a.float().cpu().numpy(), b.float().cpu().numpy(), False, True)) <= TOL
+
+
+# token rows of 1, 3, 8 and 24 vectors, of just over a power of two, of a block and of several blocks; rows beyond the last block
+@pytest.mark.parametrize("b,h,t,hd", [(3, 1, 7, 1), (2, 1, 1000, 4), (5, 2, 333, 16), (1, 3, 129, 5), (2, 1, 65, 256), (1, 43, 31, 8), (2, 25, 33, 63), (1, 1, 20000, 64)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_head_split_and_merge_of_any_width(b, h, t, hd, dt):
+    x = torch.randn(b, t, 3 * h * hd, device=DEV).to(dt)
+    q, k, v = (torch.full((b, h, t, hd), 7.0, device=DEV, dtype=dt) for _ in range(3))
+    L.head_split(q, k, v, x)
+    for i, part in enumerate((q, k, v)):
+        assert torch.equal(part, x.view(b, t, 3, h, hd)[:, :, i].transpose(1, 2))
+    y = torch.full((b, t, h * hd), 7.0, device=DEV, dtype=dt)
+    L.head_merge(y, v)
+    assert torch.equal(y, x[..., 2 * h * hd:])
