@@ -221,15 +221,16 @@ __device__ __forceinline__ float mask_sum_of_block(const float* mask, int64_t ro
 }
 
 // Per row what the dLogits epilogue of the LM-head product needs: (log-sum-exp, weight), the
-// weight being dloss * mask[r] / sum(mask).
+// weight being dloss * mask[r] / sum(mask).  A loop over rows: every block sums the mask, so there are no more of them than SMs
+// (a block per 256 rows of 2^20: 0.6 ms more).
 __global__ void __launch_bounds__(256)
 ce_grad_rows_kernel(float2* out, const float* lse, const float* mask, float dloss, int64_t rows) {
     __shared__ float sh[32];
     grid_launch_dependents();
     grid_dependency_wait();
     const float w = mask_sum_of_block<256>(mask, rows, sh);
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-    if (row < rows) out[row] = make_float2(lse[row], dloss * mask[row] / w);
+    for (int64_t row = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; row < rows; row += static_cast<int64_t>(gridDim.x) * 256)
+        out[row] = make_float2(lse[row], dloss * mask[row] / w);
 }
 
 // llmt's planned cross_entropy_bwd (docs/TODO.md:216-217): dlogits = (softmax - onehot) * mask / sum(mask),
@@ -370,8 +371,9 @@ cudaError_t launch_cross_entropy_bwd(float* dlogits, const float* logits, const 
 }
 
 cudaError_t launch_ce_grad_rows(void* out, const float* lse, const float* mask, float dloss, int64_t rows, cudaStream_t stream) {
-    return launch_dependent(ce_grad_rows_kernel, static_cast<unsigned>((rows + 255) / 256), 256, stream, static_cast<float2*>(out), lse,
-                            mask, dloss, rows);
+    const int64_t blocks = (rows + 255) / 256;
+    return launch_dependent(ce_grad_rows_kernel, static_cast<unsigned>(blocks < 148 ? blocks : 148), 256, stream, static_cast<float2*>(out),
+                            lse, mask, dloss, rows);
 }
 
 cudaError_t launch_lse_from_stats(float* lse, const void* stats, int64_t rows, int parts, cudaStream_t stream) {

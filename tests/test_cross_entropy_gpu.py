@@ -218,3 +218,22 @@ def test_lm_head_dlogits_from_the_product(m, vocab, k, out_dtype, reuse):
     dl2 = torch.full((m, ld), float("nan"), device=DEV, dtype=out_dtype)[:, :vocab]
     L.lm_head_ce_bwd(d, dl2, xd, wd, td, md, dloss=1.0, stats_valid=False)
     assert torch.equal(dl, dl2)
+
+
+def test_lm_head_dlogits_of_more_rows_than_one_pass_of_the_row_kernel():
+    """148 blocks of 256 rows and a few: every row gets its own weight (the rows are alike up to mask and target)."""
+    rows, vocab, k = 148 * 256 + 300, 64, 64
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.randn(rows, k, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(vocab, k, device=DEV, generator=g) * 0.2).bfloat16()
+    t = torch.randint(vocab, (rows,), device=DEV, generator=g, dtype=torch.int32)
+    m = torch.rand(rows, device=DEV, generator=g)
+    got = torch.empty(rows, vocab, device=DEV)
+    d = L.make_desc(got, x, w, False, True)
+    ws = torch.empty(L.lm_head_ce_workspace_bytes(d, x, w), dtype=torch.uint8, device=DEV)
+    d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+    L.lm_head_ce_bwd(d, got, x, w, t, m, 2.0)
+    p = torch.softmax(x.double() @ w.double().T, 1)
+    p[torch.arange(rows, device=DEV), t.long()] -= 1.0
+    want = p * (2.0 * m.double() / m.double().sum())[:, None]
+    assert ((got.double() - want).norm(dim=1) <= 1e-4 * want.norm(dim=1)).all()   # (exponentials and sums in fp32, the hardware's exp2)
