@@ -1,4 +1,4 @@
-"""The strict-fp32 GEMM at the edges of its tile forms, its cluster splits and its copy paths.
+"""fp32 products by FMAs at the edges of their tile forms, cluster splits and copy paths, and small ones on the tensor cores.
 
 Bound: an fp32 sum of k products in any order differs from the exact one by at most k * 2^-24 of the sum of
 magnitudes; for random signs the error grows with sqrt(k) instead.  8 sqrt(k) 2^-24 in the Frobenius norm
@@ -20,10 +20,15 @@ def _bound(k):
     return 8.0 * max(k, 1) ** 0.5 * 2.0 ** -24
 
 
-# (m, n, k): one element; tile edges +- 1; one row; k below, at and beyond a stage and a split; the 8-warp form with
-# 8-way splits; the last split empty (k = 16 * 4 * 17 over 8 splits of 3 stages); an odd pitch with many tiles
+# (m, n, k): one element; tile edges +- 1; one row; k below, at and beyond a stage and a split; the last split empty (k = 1088:
+# 34 stages over 8 splits of 5); on the tensor cores one tile in 8 splits, an odd pitch with many tiles, a long reduction
 SIZES = [(1, 1, 1), (128, 64, 16), (129, 65, 17), (63, 64, 15), (64, 63, 64), (3, 200, 300), (1, 128, 2176), (64, 64, 5000),
          (65, 130, 1088), (300, 2000, 131), (517, 771, 259), (130, 70, 22000)]
+# Every form of the FMA kernel and every number of splits that its cost model gives it without a bias gradient
+FORMS = [(462, 1176, 17, "128x64 warps=4 splits=1"), (131, 67, 70, "128x64 warps=4 splits=4"), (131, 67, 135, "128x64 warps=4 splits=8"),
+         (1030, 1042, 17, "64x64 warps=4 splits=1"), (3, 1188, 129, "64x64 warps=4 splits=4"), (65, 67, 270, "64x64 warps=4 splits=8"),
+         (67, 3, 17, "64x64 warps=8 splits=1"), (1188, 66, 194, "64x64 warps=8 splits=2"), (1158, 3, 387, "64x64 warps=8 splits=4"),
+         (3, 978, 2307, "64x64 warps=8 splits=8")]
 
 
 @pytest.mark.parametrize("m,n,k", SIZES)
@@ -47,6 +52,15 @@ def test_tiles_splits_and_pitches(m, n, k, ta, tb):
     L.gemm(cv, av, bv, bool(ta), bool(tb), alpha=0.75, beta=0.5)
     assert torch.equal(cv, c), "the copy path does not change the sums"
     assert bool((cf[:, 0] == 7.0).all()) and bool((cf[:, 1 + n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,n,k,form", FORMS)
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_every_form_of_the_fma_kernel(m, n, k, form, ta, tb):
+    a = np.empty((k, m) if ta else (m, k), dtype=np.float32)
+    b = np.empty((n, k) if tb else (k, n), dtype=np.float32)
+    assert f"fp32-simt tile={form} " in L.plan(L.make_desc(torch.empty(m, n), torch.from_numpy(a), torch.from_numpy(b), bool(ta), bool(tb)))
+    test_tiles_splits_and_pitches(m, n, k, ta, tb)
 
 
 @pytest.mark.parametrize("ta", [0, 1])
