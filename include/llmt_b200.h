@@ -89,13 +89,15 @@ enum llmt_b200_status {
  *                m, n, k and batch must be below 2^31 - 1024.
  *   stride_*     elements between consecutive batch items; ignored when batch == 1.
  *   dtype_ab     element type of A and B; dtype_c of C.  Supported pairs:
- *                (fp32, fp32) strict fp32 FMA path; (bf16, bf16) and (bf16, fp32)
+ *                (fp32, fp32) at fp32 precision (never TF32): FMAs for small problems, for the
+ *                others three bf16 parts per value on the tensor cores, the parts' sums added
+ *                in fp32 (llmt_b200_gemm_plan says which); (bf16, bf16) and (bf16, fp32)
  *                tensor-core path with fp32 accumulation.
  *   bias         [n] values added to every row when EPI_BIAS is set (bias_dtype: fp32 or bf16).
  *   dbias        optional fp32 [m]:  dbias[i] = dbias_beta * dbias[i] + sum_p op(A)[i,p].
  *                For llmt's dW call (src/layers/linear.cpp:27-29: A = dy, trans_a = 1)
  *                this is the bias gradient, summed over tokens, in a fixed order, by the same
- *                launch that computes dW (on the strict-fp32 path: by a second small kernel).
+ *                launch that computes dW.
  *   Aliasing     C is read and written in place.  C, dbias and the workspace must not overlap
  *                one another, A, B or bias (checked by address range).
  *   plan_*       tuning overrides of the tile width, split-K factor and CTA pairing; 0 leaves the
@@ -236,8 +238,9 @@ LLMT_B200_API int llmt_b200_device_status(int32_t* code, int32_t* detail);
 
 /* How long a wait inside a kernel may last before it gives up, in nanoseconds: gemm_ns for
  * the GEMM kernels' barrier waits (default 2 s), exchange_ns for the gradient exchange's
- * waits on its peers (default 4 s); 0 leaves a value as it is.  Applies to launches made
- * after the call.  Meant for tests and for hosts with their own watchdog period. */
+ * waits on its peers (default 4 s); 0 leaves a value as it is.  An fp32 product on the tensor
+ * cores adds 2 us per k of a split to gemm_ns: sums with operands that are not finite are
+ * formed a second time while the other warps wait.  Applies to launches made after the call.  Meant for tests and for hosts with their own watchdog period. */
 LLMT_B200_API int llmt_b200_set_wait_limit_ns(uint64_t gemm_ns, uint64_t exchange_ns);
 
 /* Host-side cache of encoded TMA descriptors (the counterpart of llmt's AlgoCache,
@@ -253,7 +256,8 @@ LLMT_B200_API void llmt_b200_tensor_map_cache_stats(uint64_t* hits, uint64_t* mi
 LLMT_B200_API int llmt_b200_zero_grads(float* span, int64_t count, void* stream);
 
 /* SMs the persistent GEMM kernels may occupy from now on: 0 (the default) = every SM.
- * Planning and grid size follow it.  A data-parallel caller lowers it by the number of
+ * Planning and grid size follow it (fp32 products by FMAs run short CTAs on whatever SM is
+ * free; their plan follows it too).  A data-parallel caller lowers it by the number of
  * CTAs its collective library runs (e.g. 148 - 8), so that the all-reduce of one layer's
  * gradients, enqueued on a second stream, finds free SMs while the next layer's GEMM
  * launch is resident.  Returns the previous value, or a negative value for sms < 0.

@@ -77,7 +77,7 @@ struct Tensor {
 };
 
 // {master, gemm_compute, reduce} (llmt precision.h:16-22).  Two settings have
-// kernels: fp32() = strict fp32 FMA, and bf16_mixed() = bf16 tensor-core
+// kernels: fp32() = fp32 precision throughout, and bf16_mixed() = bf16 tensor-core
 // multiply with fp32 accumulation.
 struct PrecisionPolicy {
     DType master = DType::FP32;

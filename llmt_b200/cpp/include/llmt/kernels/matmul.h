@@ -9,7 +9,7 @@ namespace llmt::kernels {
 
 // C[M,N] = alpha*op(A)*op(B) + beta*C for row-major tensors; rank 2 = one GEMM,
 // rank 3 = one independent GEMM per leading index.  Same contract, same abort
-// messages as llmt.  dtype rules: all fp32 (strict fp32 path, needs
+// messages as llmt.  dtype rules: all fp32 (fp32 precision, never TF32; needs
 // ctx.precision == fp32()), or A/B bf16 with C bf16 or fp32 (tensor-core path,
 // needs gemm_compute == BF16, reduce == FP32).
 void matmul(const RunCtx& ctx, Tensor& c, const Tensor& a, const Tensor& b, bool trans_a,
