@@ -16,11 +16,11 @@
 // Products with few tiles and a long reduction are split along k over the CTAs of a cluster, which add their
 // partial tiles through distributed shared memory in rank order: no scratch, no second launch, one fixed order.
 //
-// Bound: the shared-memory data pipe.  Counted in 128-byte wavefronts per k-block of a 128 x 128 tile: 2304 for the MMAs'
-// operands (an MMA of 128 x 128 x 16 reads A once and B twice: 96 wavefronts for 64 cycles of arithmetic), 768 for
-// the parts' stores, 512 for the loads: 3584, measured 3300-3800 cycles.  A CTA pair (256 x 128 tiles, half of B each) and
-// sixteen splitting warps with half the registers measured the same.  BN = 64 takes 2500 cycles for half the outputs and
-// serves problems with few tiles.
+// Bound: the SM's L1 and shared-memory data pipe.  Counters of 2048 x 4096 x 2048, per k-block of a 128 x 128 tile: 1536
+// wavefronts for the MMAs' operands (an MMA of 128 x 128 x 16 takes 64), 1071 for the parts' stores and the epilogue (197 of
+// them bank conflicts), 826 for the loads: 3433, in 3540 active cycles, 97 %.  A CTA pair (256 x 128 tiles, half of B
+// each) and sixteen splitting warps with half the registers measured the same.  BN = 64 takes 2500 cycles for half the
+// outputs and serves problems with few tiles.
 //
 // Measured against the FMA kernel (us, and error against 64 bits): y = x W^T 256 x 3072 x 768 36.8 -> 20.7 (2.5e-7 ->
 // 1.0e-7), 512 x 50257 x 768 856 -> 294 (5.0e-7 -> 1.0e-7), dX of that layer 962 -> 402 (1.4e-6 -> 2.7e-7), its dW
