@@ -712,7 +712,8 @@ cudaError_t launch_fp32_tc(const Fp32GemmParams& in, const Fp32Plan& plan, cudaS
     p.vec_c = aligned(p.c, p.ldc, p.stride_c, p.stride_c_outer);
     // While a tile's sums are formed again by FMAs (at most 0.6 us per k, measured) the CTA's other warps wait for it: that time comes
     // on top of what a caller allows a wait to take.
-    p.wait_limit_ns += static_cast<uint64_t>(p.k_per_split) * 2000u;
+    const uint64_t more = static_cast<uint64_t>(p.k_per_split) * 2000u;
+    p.wait_limit_ns = p.wait_limit_ns < UINT64_MAX - more ? p.wait_limit_ns + more : UINT64_MAX;
     const unsigned grid = static_cast<unsigned>(plan.ctas);
     return plan.bn == 128 ? launch_tc_size<128>(p, grid, stream) : launch_tc_size<64>(p, grid, stream);
 }

@@ -209,16 +209,17 @@ def test_sums_formed_again_by_fmas(m, n, k, ta, tb):
     assert _rel(c[1:m - 1, :n - 1][:, -64:], ref[1:m - 1, :n - 1][:, -64:]) <= 8.0 * k ** 0.5 * 2.0 ** -24
 
 
-def test_a_short_wait_limit_allows_for_sums_formed_again():
+@pytest.mark.parametrize("limit_ns", [500000, 2 ** 64 - 1])
+def test_a_short_wait_limit_allows_for_sums_formed_again(limit_ns):
     """25000 k per split take milliseconds when they are formed again by FMAs, with the other warps waiting: no reason to give up,
-    also where a caller allows a wait half a millisecond."""
+    also where a caller allows a wait half a millisecond, or as long as it can say."""
     k = 200000
     a, b = _operands(128, 128, k, 0, 1)
     a[5, 7] = float("nan")
     c = torch.empty(128, 128, device=DEV)
     L.gemm(c, a, b, False, True)
     torch.cuda.synchronize()
-    L.set_wait_limit_ns(gemm_ns=500000)
+    L.set_wait_limit_ns(gemm_ns=limit_ns)
     try:
         L.gemm(c, a, b, False, True)
         assert L.device_status() == (0, 0)
